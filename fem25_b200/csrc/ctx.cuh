@@ -64,6 +64,15 @@ struct PairTable {
   double2 p[kMaxPairs];
 };
 
+// 1D Lagrange factors of the element's shape functions at the 13 points:
+// l[q][i] = l_i(x_q), d[q][i] = l_i'(x_q)  (SHL = l(xi) l(eta), dshl.f:100-243);
+// passed to the gradient kernels by value
+struct ShapeTabs {
+  double l[kNint][kNl];
+  double d[kNint][kNl];
+};
+ShapeTabs shape_tables(const Tables &t);
+
 // Options of the misfit / adjoint source (the reference's INV_INFO fields
 // NORM, IRESTP, IBPHASE, the thresholds of COBJ4 and the DTMAX phase-jump
 // tests), and the per-call values the kernel needs.
@@ -113,7 +122,7 @@ struct Ctx {
   double *d_prim = nullptr;      // [nzero] K0/K1 basis value of every CSR entry
   unsigned *d_desc = nullptr;    // [nzero] block << 4 | i << 2 | j
   int stream_variant = -1;       // loop order of the streaming kernel (-1: not tuned yet)
-  int grad_tile = -1;            // source tile of the FP64 gradient (-1: not tuned yet)
+  int grad_tile = -1;            // field tile of the last FP64 gradient (-1: none yet)
   double *d_ebasis = nullptr;    // [nelem][625][12] scratch
   int *d_bgptr = nullptr, *d_bglist = nullptr;  // block -> (element node pair) ids
   bool basis_valid = false;

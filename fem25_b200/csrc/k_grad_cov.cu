@@ -727,13 +727,6 @@ constexpr int kSmemDoubles = 2 * kRaw + 2 * kZ + 4 * kW + 2 * kNint * kNl + 4 * 
 constexpr int kSmemBytes = kSmemDoubles * 8;  // 72 KB: three CTAs per SM
 }  // namespace covf
 
-// 1D Lagrange factors of the element's shape functions at the 13 points:
-// l[q][i] = l_i(x_q), d[q][i] = l_i'(x_q)  (SHL = l(xi) l(eta), dshl.f:100-243)
-struct CovFinTabs {
-  double l[kNint][kNl];
-  double d[kNint][kNl];
-};
-
 // raw blocks behind combined block b (stored [j][i]): first index and count
 __device__ __forceinline__ void cov_raw_of(int b, int *ids, int &n) {
   switch (b) {
@@ -778,7 +771,7 @@ __device__ __forceinline__ double cov_fw(const double *W, int qz, const double *
 
 __global__ void __launch_bounds__(covf::kThreads, 3)
     k_grad_cov_fin(MeshView mv, DevTables dt, int n_elem, int nnpg, const int *__restrict__ elems,
-                   const double *__restrict__ accb, CovFinTabs tb, double *__restrict__ grad,
+                   const double *__restrict__ accb, ShapeTabs tb, double *__restrict__ grad,
                    int *__restrict__ err) {
   extern __shared__ __align__(16) double fs[];
   double *rawb = fs;                          // [2][kRaw]
@@ -972,29 +965,6 @@ __global__ void __launch_bounds__(covf::kThreads, 3)
 // ---------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------
-static CovFinTabs cov_fin_tables(const Tables &t) {
-  // Lagrange basis on the 5 GLL points (the factors of SHL, dshl.f:100-243)
-  CovFinTabs tb;
-  for (int q = 0; q < kNint; q++) {
-    const double x = t.xigll[q];
-    for (int i = 0; i < kNl; i++) {
-      double v = 1.0, dsum = 0.0;
-      for (int k = 0; k < kNl; k++)
-        if (k != i) v *= (x - t.xipts[k]) / (t.xipts[i] - t.xipts[k]);
-      for (int m = 0; m < kNl; m++) {
-        if (m == i) continue;
-        double p = 1.0 / (t.xipts[i] - t.xipts[m]);
-        for (int k = 0; k < kNl; k++)
-          if (k != i && k != m) p *= (x - t.xipts[k]) / (t.xipts[i] - t.xipts[k]);
-        dsum += p;
-      }
-      tb.l[q][i] = v;
-      tb.d[q][i] = dsum;
-    }
-  }
-  return tb;
-}
-
 // Gather plan of the covariance accumulation for every element outside the
 // PML (kernel order): the element's nodes, sorted by first DOF.  An element
 // whose 25 nodes are one run of 20 consecutive nodes plus five nodes
@@ -1198,7 +1168,7 @@ cudaError_t launch_grad_cov_fin(Ctx *c, double *grad, cudaStream_t st) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
   const int grid = std::min(3 * nsm, c->n_nonpml);
   k_grad_cov_fin<<<grid, covf::kThreads, covf::kSmemBytes, st>>>(
-      c->mv, c->dt, c->n_nonpml, c->nnpg, c->d_nonpml, c->d_cov, cov_fin_tables(c->tab), grad,
+      c->mv, c->dt, c->n_nonpml, c->nnpg, c->d_nonpml, c->d_cov, shape_tables(c->tab), grad,
       c->d_err);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) c->cov_pending = false;
