@@ -36,6 +36,7 @@ UNITS = [
     ("misfit_noalloc.cu", ["-fmad=false"]),
     ("dense_solve.cu", []),
     ("sparse_solve.cu", []),
+    ("sparse_factor.cu", []),
 ]
 HOST = [("host_setup.cpp", ["-O2", "-ffp-contract=off", "-fPIC", "-fopenmp", "-std=c++17"]),
         ("mesh_io.cpp", ["-O2", "-ffp-contract=off", "-fPIC", "-std=c++17"])]

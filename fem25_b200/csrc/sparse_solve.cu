@@ -16,93 +16,31 @@
 // summed" rows and columns, eliminated there) and its boundary: the DOFs of
 // its subtree's elements owned by an ancestor, ordered by elimination.
 //
-// Factorisation (device), level by level from the leaves: every front of a
-// level is assembled in a work buffer -- the CSR entries whose first
-// eliminated DOF it owns, plus the update (Schur complement) blocks of its
-// two children (extend-add) -- and partially factored: F11 = P L11 U11 with
-// partial pivoting restricted to the fully summed rows, L21 = F21 U11^-1,
-// U12 = L11^-1 P F12, update = F22 - L21 U12.  Fronts up to kSmallN rows are
-// factored one CTA each in a single launch per level (blocked by panels of
-// kNb columns factored in shared memory, rank-kNb trailing updates); larger
-// fronts (the top levels of the tree) go to cuSOLVER getrf and cuBLAS trsm /
-// gemm.  The factors (L11\U11 over L21, and U12) are copied to a store kept
-// by the context; the update blocks live until the parent level has consumed
+// Factorisation (device, sparse_factor.cu), level by level from the leaves: every
+// front of a level is assembled in a work buffer -- the update (Schur complement)
+// blocks of its two children, plus the CSR entries whose first eliminated DOF it
+// owns -- and partially factored: F11 = P L11 U11 with partial pivoting
+// restricted to the fully summed rows, L21 = F21 U11^-1, U12 = L11^-1 P F12,
+// update = F22 - L21 U12.  The factors (L11\U11 over L21, and U12) go to a store
+// kept by the context; the update blocks live until the parent level has consumed
 // them (two work buffers, alternating).
 //
 // Solve (device), one launch per level: forward elimination from the leaves,
 // back substitution from the root, for op(A) = A, A^T (MUMPS ICNTL(9) != 1)
-// or A^H; a CTA per (front, group of right-hand sides), the triangles solved
-// in blocks of 32 rows.
-#include <cublas_v2.h>
-#include <cusolverDn.h>
-
+// or A^H; a CTA per (front, group of right-hand sides), the triangles in
+// blocks of 32 rows whose diagonal blocks the store holds inverted.
 #include <algorithm>
 #include <cstdio>
 #include <numeric>
 
-#include "ctx.cuh"
+#include "sparse.cuh"
 
 namespace fem25 {
 
-namespace sp {
-constexpr int kLeafElems = 2;     // elements per leaf of the dissection
-constexpr int kSmallN = 1024;     // fronts up to this many rows: one CTA each
-constexpr int kNb = 8;            // panel width of the one-CTA factorisation
-constexpr int kFacThreads = 256;  // threads of the one-CTA factorisation (128 measured slower)
+namespace {
 constexpr int kThreads = 256;
-constexpr int kRhsPerCta = 8;     // right-hand sides per solve CTA
-constexpr int kLanes = 8;         // streams for the library-factored fronts of a level
-}  // namespace sp
-
-struct SpFront {
-  int k, m;             // own (fully summed) and boundary DOFs
-  int parent;           // -1: root
-  int child[2];         // -1: none
-  int level;            // depth in the dissection tree (root 0)
-  long long own0;       // first own DOF in own[] (= elimination position)
-  long long bnd0;       // first boundary DOF in bnd[]
-  long long ea0;        // first entry of its extend-add map (ea[], m entries)
-  long long fac0;       // factor store: L block [n][k] (ld n), then U12 [k][m] (ld k)
-  long long work0;      // offset of its n x n front in its level's work buffer
-};
-
-// one stream of the library path with its own handles and workspace
-struct SpLane {
-  cudaStream_t st = nullptr;
-  cudaEvent_t done = nullptr;
-  cusolverDnHandle_t sol = nullptr;
-  cusolverDnParams_t par = nullptr;
-  cublasHandle_t blas = nullptr;
-  void *dwork = nullptr;
-  size_t dwork_bytes = 0;
-  std::vector<char> hwork;
-  int *d_getrf_info = nullptr;
-};
-
-struct SparseLU {
-  bool analysed = false, factored = false;
-  int nfront = 0, nlevel = 0;
-  std::vector<SpFront> fr;
-  std::vector<std::vector<int>> lev;        // front ids per level, one-CTA fronts first
-  std::vector<int> lev_nsmall, lev_nmax_small;  // per level: one-CTA fronts, their largest order
-  std::vector<int> lev_kmax, lev_mmax;          // per level: largest own and boundary counts
-  std::vector<long long> lev_work;          // work elements per level
-  std::vector<long long> lev_ent0;          // first CSR-entry record of each level
-  long long fac_elems = 0, max_work = 0;
-  // device
-  SpFront *d_fr = nullptr;
-  int *d_own = nullptr, *d_bnd = nullptr, *d_ea = nullptr;
-  int *d_lev_fronts = nullptr;              // all levels' front ids, concatenated
-  std::vector<long long> lev_off;           // offset of each level in d_lev_fronts
-  int *d_ent_idx = nullptr;                 // CSR entries by level, and their
-  long long *d_ent_loc = nullptr;           // offsets in the level's work buffer
-  double2 *d_fac = nullptr;                 // factor store
-  int64_t *d_piv = nullptr;                 // pivots (1-based within each front), [NDOF]
-  double2 *d_work[2] = {nullptr, nullptr};
-  int *d_info = nullptr;                    // first zero pivot (front + 1), 0 = none
-  SpLane lane[sp::kLanes];
-  cudaEvent_t level_ready = nullptr;
-};
+constexpr int kRhsPerCta = 8;  // right-hand sides per solve CTA
+}  // namespace
 
 // ---------------------------------------------------------------------------
 // symbolic analysis (host)
@@ -207,7 +145,7 @@ struct FrontPlan {
   std::vector<int> owner;
   std::vector<std::vector<int>> lev;
   std::vector<long long> lev_work;
-  long long fac_elems = 0, bnd_tot = 0;
+  long long fac_elems = 0, bnd_tot = 0, map_tot = 0;
   int nlev = 0;
 };
 
@@ -277,8 +215,9 @@ static int plan_fronts(int nelem, int n, const int *lm, const int *ieng, const d
     SpFront &f = b.fr[t];
     const long long nn = (long long)f.k + f.m;
     f.bnd0 = bnd_tot;
-    f.ea0 = bnd_tot;
     bnd_tot += f.m;
+    f.map0 = pl->map_tot;
+    pl->map_tot += 2 * nn;
     f.fac0 = fac;
     fac += nn * f.k + (long long)f.k * f.m;
     f.work0 = pl->lev_work[f.level];
@@ -363,19 +302,26 @@ static int sparse_analyse(Ctx *c, SparseLU *s, cudaStream_t st, std::string *msg
   s->max_work = 0;
   for (long long w : s->lev_work) s->max_work = std::max(s->max_work, w);
   const long long bnd_tot = pl.bnd_tot;
-  // extend-add maps: child boundary DOF -> index in the parent's front
-  std::vector<int> ea(bnd_tot), own_all(n), bnd_all(bnd_tot);
+  // pull maps: index in a front -> index in the boundary of child 0 / 1, or -1
+  std::vector<int> pull(pl.map_tot, -1), own_all(n), bnd_all(bnd_tot);
   for (int t = 0; t < nf; t++) {
     const SpFront &f = b.fr[t];
     std::copy(b.own_list[t].begin(), b.own_list[t].end(), own_all.begin() + f.own0);
     std::copy(bnd[t].begin(), bnd[t].end(), bnd_all.begin() + f.bnd0);
+    if (f.m > 0 && f.parent < 0) {
+      *msg = "sparse solve: a boundary DOF has no parent front";
+      return FEM25_ERR_PATTERN;
+    }
+    if (f.m == 0) continue;
+    const SpFront &pf = b.fr[f.parent];
+    int *map = pull.data() + pf.map0 + (pf.child[0] == t ? 0 : (long long)pf.k + pf.m);
     for (int i = 0; i < f.m; i++) {
-      const int li = f.parent >= 0 ? local(f.parent, bnd[t][i]) : -1;
+      const int li = local(f.parent, bnd[t][i]);
       if (li < 0) {
         *msg = "sparse solve: a boundary DOF is missing from the parent front";
         return FEM25_ERR_PATTERN;
       }
-      ea[f.ea0 + i] = li;
+      map[li] = i;
     }
   }
   // CSR entries -> (front, local offset), grouped by level
@@ -439,24 +385,27 @@ static int sparse_analyse(Ctx *c, SparseLU *s, cudaStream_t st, std::string *msg
     return FEM25_ERR_PATTERN;
   }
   std::vector<int>().swap(jc);
-  // one-CTA fronts first in each level's list
+  // fronts with k <= kSmallK first in each level's list
   s->lev_nsmall.assign(nlev, 0);
-  s->lev_nmax_small.assign(nlev, 0);
+  s->lev_ksmall.assign(nlev, 0);
+  s->lev_msmall.assign(nlev, 0);
   s->lev_kmax.assign(nlev, 0);
   s->lev_mmax.assign(nlev, 0);
-  for (int t = 0; t < nf; t++) {
-    s->lev_kmax[b.fr[t].level] = std::max(s->lev_kmax[b.fr[t].level], b.fr[t].k);
-    s->lev_mmax[b.fr[t].level] = std::max(s->lev_mmax[b.fr[t].level], b.fr[t].m);
-  }
+  s->lev_nmax.assign(nlev, 0);
+  auto small = [&](int t) { return b.fr[t].k <= sp::kSmallK; };
   for (int l = 0; l < nlev; l++) {
-    std::stable_partition(s->lev[l].begin(), s->lev[l].end(), [&](int t) {
-      return b.fr[t].k + b.fr[t].m <= sp::kSmallN;
-    });
-    for (int t : s->lev[l])
-      if (b.fr[t].k + b.fr[t].m <= sp::kSmallN) {
+    std::stable_partition(s->lev[l].begin(), s->lev[l].end(), small);
+    for (int t : s->lev[l]) {
+      const SpFront &f = b.fr[t];
+      s->lev_kmax[l] = std::max(s->lev_kmax[l], f.k);
+      s->lev_mmax[l] = std::max(s->lev_mmax[l], f.m);
+      s->lev_nmax[l] = std::max(s->lev_nmax[l], f.k + f.m);
+      if (small(t)) {
         s->lev_nsmall[l]++;
-        s->lev_nmax_small[l] = std::max(s->lev_nmax_small[l], b.fr[t].k + b.fr[t].m);
+        s->lev_ksmall[l] = std::max(s->lev_ksmall[l], f.k);
+        s->lev_msmall[l] = std::max(s->lev_msmall[l], f.m);
       }
+    }
   }
   // level front lists, concatenated
   std::vector<int> lf;
@@ -475,7 +424,7 @@ static int sparse_analyse(Ctx *c, SparseLU *s, cudaStream_t st, std::string *msg
   if ((e = up((void **)&s->d_fr, b.fr.data(), sizeof(SpFront) * nf)) ||
       (e = up((void **)&s->d_own, own_all.data(), sizeof(int) * n)) ||
       (e = up((void **)&s->d_bnd, bnd_all.data(), sizeof(int) * bnd_tot)) ||
-      (e = up((void **)&s->d_ea, ea.data(), sizeof(int) * bnd_tot)) ||
+      (e = up((void **)&s->d_pull, pull.data(), sizeof(int) * pull.size())) ||
       (e = up((void **)&s->d_lev_fronts, lf.data(), sizeof(int) * lf.size())) ||
       (e = up((void **)&s->d_ent_idx, sidx.data(), sizeof(int) * sidx.size())) ||
       (e = up((void **)&s->d_ent_loc, sloc.data(), sizeof(long long) * sloc.size()))) {
@@ -488,232 +437,6 @@ static int sparse_analyse(Ctx *c, SparseLU *s, cudaStream_t st, std::string *msg
   s->analysed = true;
   (void)st;
   return 0;
-}
-
-// ---------------------------------------------------------------------------
-// numeric factorisation (device)
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cfms(double2 acc, double2 a, double2 b) {  // acc - a b
-  return make_double2(acc.x - a.x * b.x + a.y * b.y, acc.y - a.x * b.y - a.y * b.x);
-}
-__device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
-  const double d = b.x * b.x + b.y * b.y;
-  return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
-}
-__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-
-// CSR entries of one level into their fronts' work buffers
-__global__ void k_sp_assemble(long long n, const int *__restrict__ idx,
-                              const long long *__restrict__ loc, const double2 *__restrict__ csr,
-                              double2 *__restrict__ work) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    work[loc[i]] = csr[idx[i]];
-}
-
-// extend-add of child slot `slot` of every front of the level: one CTA per front
-__global__ void k_sp_extend_add(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
-                                const int *__restrict__ ea, const double2 *__restrict__ wchild,
-                                double2 *__restrict__ work, int slot) {
-  const SpFront f = fr[fronts[blockIdx.x]];
-  const int ch = f.child[slot];
-  if (ch < 0) return;
-  const SpFront g = fr[ch];
-  const long long nf = (long long)f.k + f.m, ng = (long long)g.k + g.m;
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int j = blockIdx.y * nw + (threadIdx.x >> 5); j < g.m; j += gridDim.y * nw) {
-    const double2 *src = wchild + g.work0 + g.k + (long long)(g.k + j) * ng;
-    double2 *dst = work + f.work0 + (long long)ea[g.ea0 + j] * nf;
-    for (int i = lane; i < g.m; i += 32) {
-      const double2 v = src[i];
-      double2 *o = dst + ea[g.ea0 + i];
-      o->x += v.x;
-      o->y += v.y;
-    }
-  }
-}
-
-// Partial LU of one front per CTA, blocked by panels of kNb columns: the
-// panel (rows jb..n-1) is factored in shared memory with partial pivoting
-// restricted to the fully summed rows, its row interchanges are applied to
-// the front's other columns, the panel's U block (rows jb..jb+nb-1) is
-// solved with the panel's unit lower triangle, and the trailing block is
-// updated by a rank-nb product: a warp per pair of columns, their U values
-// in registers, the panel rows read from shared memory.  In place in the
-// work buffer; pivots 1-based within the front.
-__global__ void __launch_bounds__(sp::kFacThreads) k_sp_factor_blk(
-    const int *__restrict__ fronts, int nfr, const SpFront *__restrict__ fr,
-    double2 *__restrict__ work, int64_t *__restrict__ piv, int *__restrict__ info) {
-  extern __shared__ double2 P[];  // panel: P[r + c * pr], r < pr = n - jb, c < nb
-  __shared__ double red_v[sp::kFacThreads / 32];
-  __shared__ int red_i[sp::kFacThreads / 32];
-  __shared__ int swp[sp::kNb];
-  const int b = blockIdx.x;
-  if (b >= nfr) return;
-  const int t = fronts[b];
-  const SpFront f = fr[t];
-  const int k = f.k, n = f.k + f.m;
-  double2 *F = work + f.work0;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)(blockDim.x >> 5);
-  for (int jb = 0; jb < k; jb += sp::kNb) {
-    const int nb = min(sp::kNb, k - jb), pr = n - jb, kr = k - jb;
-    // 1. the panel to shared memory
-    for (int c = 0; c < nb; c++)
-      for (int r = tid; r < pr; r += blockDim.x) P[r + c * pr] = F[jb + r + (long long)(jb + c) * n];
-    __syncthreads();
-    // 2. unblocked LU of the panel; pivots among its first kr rows
-    for (int j = 0; j < nb; j++) {
-      double best = -1.0;
-      int bi = j;
-      for (int r = j + tid; r < kr; r += blockDim.x) {
-        const double2 v = P[r + j * pr];
-        const double a = fabs(v.x) + fabs(v.y);
-        if (a > best) {
-          best = a;
-          bi = r;
-        }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (lane == 0) {
-        red_v[warp] = best;
-        red_i[warp] = bi;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double bb = -1.0;
-        int ii = j;
-        for (int w = 0; w < nw; w++)
-          if (red_v[w] > bb || (red_v[w] == bb && red_i[w] < ii)) {
-            bb = red_v[w];
-            ii = red_i[w];
-          }
-        swp[j] = ii;
-        piv[f.own0 + jb + j] = jb + ii + 1;
-        if (bb <= 0.0) atomicCAS(info, 0, t + 1);
-      }
-      __syncthreads();
-      const int pj = swp[j];
-      if (pj != j)
-        for (int c = tid; c < nb; c += blockDim.x) {
-          const double2 x = P[j + c * pr];
-          P[j + c * pr] = P[pj + c * pr];
-          P[pj + c * pr] = x;
-        }
-      __syncthreads();
-      const double2 d = P[j + j * pr];
-      const bool zero = d.x == 0.0 && d.y == 0.0;
-      for (int r = j + 1 + tid; r < pr; r += blockDim.x)
-        P[r + j * pr] = zero ? make_double2(0.0, 0.0) : cdiv(P[r + j * pr], d);
-      __syncthreads();
-      for (int c = j + 1; c < nb; c++) {
-        const double2 u = P[j + c * pr];
-        for (int r = j + 1 + tid; r < pr; r += blockDim.x)
-          P[r + c * pr] = cfms(P[r + c * pr], P[r + j * pr], u);
-      }
-      __syncthreads();
-    }
-    // 3. the panel back; 4. its interchanges on the other columns
-    for (int c = 0; c < nb; c++)
-      for (int r = tid; r < pr; r += blockDim.x) F[jb + r + (long long)(jb + c) * n] = P[r + c * pr];
-    for (int c = tid; c < n - nb; c += blockDim.x) {
-      double2 *col = F + (long long)(c < jb ? c : c + nb) * n + jb;
-      for (int j = 0; j < nb; j++) {
-        const int pj = swp[j];
-        if (pj != j) {
-          const double2 x = col[j];
-          col[j] = col[pj];
-          col[pj] = x;
-        }
-      }
-    }
-    __syncthreads();
-    // 5. the U block: unit lower solve with the panel's top nb x nb triangle
-    for (int cc = jb + nb + tid; cc < n; cc += blockDim.x) {
-      double2 *col = F + (long long)cc * n + jb;
-      double2 x[sp::kNb];
-#pragma unroll
-      for (int i = 0; i < sp::kNb; i++) x[i] = i < nb ? col[i] : make_double2(0.0, 0.0);
-#pragma unroll
-      for (int i = 1; i < sp::kNb; i++)
-#pragma unroll
-        for (int j = 0; j < i; j++) x[i] = cfms(x[i], P[i + j * pr], x[j]);
-#pragma unroll
-      for (int i = 0; i < sp::kNb; i++)
-        if (i < nb) col[i] = x[i];
-    }
-    __syncthreads();
-    // 6. trailing update, rows and columns from jb + nb: a warp per pair of
-    // columns (each panel value read from shared memory feeds two columns)
-    const int c0 = jb + nb;
-    for (int cp = c0 + 2 * warp; cp < n; cp += 2 * nw) {
-      const bool two = cp + 1 < n;
-      double2 u0[sp::kNb], u1[sp::kNb];
-#pragma unroll
-      for (int j = 0; j < sp::kNb; j++) {
-        u0[j] = j < nb ? F[jb + j + (long long)cp * n] : make_double2(0.0, 0.0);
-        u1[j] = (two && j < nb) ? F[jb + j + (long long)(cp + 1) * n] : make_double2(0.0, 0.0);
-      }
-      double2 *col0 = F + (long long)cp * n, *col1 = col0 + n;
-      for (int r = c0 + lane; r < n; r += 32) {
-        double2 a0 = col0[r], a1 = two ? col1[r] : make_double2(0.0, 0.0);
-        const double2 *pl = P + (r - jb);
-#pragma unroll
-        for (int j = 0; j < sp::kNb; j++) {
-          const double2 l = j < nb ? pl[j * pr] : make_double2(0.0, 0.0);
-          a0 = cfms(a0, l, u0[j]);
-          a1 = cfms(a1, l, u1[j]);
-        }
-        col0[r] = a0;
-        if (two) col1[r] = a1;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// a library-factored front's zero pivot into the status word
-__global__ void k_sp_getrf_status(const int *getrf_info, int *info, int front) {
-  if (*getrf_info > 0) atomicCAS(info, 0, front + 1);
-}
-
-// row interchanges of a front's pivots on columns [c0, c1) (laswp)
-__global__ void k_sp_laswp(double2 *F, int n, int k, int c0, int c1, const int64_t *piv) {
-  for (int cidx = c0 + blockIdx.x * blockDim.x + threadIdx.x; cidx < c1;
-       cidx += gridDim.x * blockDim.x)
-    for (int j = 0; j < k; j++) {
-      const int p = (int)piv[j] - 1;
-      if (p != j) {
-        double2 *a = F + j + (long long)cidx * n, *b = F + p + (long long)cidx * n;
-        const double2 x = *a;
-        *a = *b;
-        *b = x;
-      }
-    }
-}
-
-// factors of the level's fronts to the store: the first k columns (L11\U11
-// over L21, n x k) and U12 (rows 0..k-1 of columns k..n-1, k x m, ld k)
-__global__ void k_sp_store(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
-                           const double2 *__restrict__ work, double2 *__restrict__ fac) {
-  const SpFront f = fr[fronts[blockIdx.x]];
-  const long long n = (long long)f.k + f.m;
-  const double2 *F = work + f.work0;
-  double2 *L = fac + f.fac0, *U = L + n * f.k;
-  const long long stride = (long long)gridDim.y * blockDim.x;
-  for (long long q = blockIdx.y * blockDim.x + threadIdx.x; q < n * f.k; q += stride) L[q] = F[q];
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int j = blockIdx.y * nw + (threadIdx.x >> 5); j < f.m; j += gridDim.y * nw)
-    for (int i = lane; i < f.k; i += 32) U[i + (long long)j * f.k] = F[i + (f.k + j) * n];
 }
 
 // ---------------------------------------------------------------------------
@@ -738,7 +461,7 @@ struct SolveArgs {
   const SpFront *fr;
   const int *own, *bnd;
   const double2 *fac;
-  const int64_t *piv;
+  const int *swap;
   double2 *x;
   int ndof, nrhs, trans;  // trans 0: A, 1: A^T, 2: A^H
 };
@@ -754,7 +477,7 @@ __device__ __forceinline__ double2 sp_el(const double2 *T, long long n, int i, i
 }
 
 template <int R>
-__global__ void __launch_bounds__(sp::kThreads) k_sp_solve_fwd(SolveArgs a) {
+__global__ void __launch_bounds__(kThreads) k_sp_solve_fwd(SolveArgs a) {
   __shared__ double2 xs[32][R];
   __shared__ double2 tb[32][33];  // the block's diagonal triangle, op applied
   const SpFront f = a.fr[a.fronts[blockIdx.x]];
@@ -769,7 +492,7 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_fwd(SolveArgs a) {
   if (tr == 0 && tid < nr) {  // row interchanges of P
     double2 *xr = x + (long long)tid * a.ndof;
     for (int j = 0; j < k; j++) {
-      const int p = (int)a.piv[f.own0 + j] - 1;
+      const int p = a.swap[f.own0 + j];
       if (p != j) {
         const double2 t = xr[ow[j]];
         xr[ow[j]] = xr[ow[p]];
@@ -784,7 +507,7 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_fwd(SolveArgs a) {
     for (int q = tid; q < nb * nb; q += blockDim.x) {
       const int i = q % nb, j = q / nb;
       if (i > j) tb[i][j] = sp_el(F, n, jb + i, jb + j, tr);
-      if (i == j && tr != 0) tb[i][i] = cdiv(make_double2(1.0, 0.0), sp_el(F, n, jb + i, jb + i, tr));
+      if (i == j) tb[i][i] = tr != 0 ? sp_el(F, n, jb + i, jb + i, tr) : make_double2(1.0, 0.0);
     }
     __syncthreads();
     if (warp == 0) {
@@ -792,20 +515,20 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_fwd(SolveArgs a) {
 #pragma unroll
       for (int s = 0; s < R; s++)
         v[s] = (lane < nb && s < nr) ? x[(long long)s * a.ndof + ow[jb + lane]] : make_double2(0.0, 0.0);
-      for (int i = 0; i < nb; i++) {
-        if (tr != 0 && lane == i) {
-          const double2 d = tb[i][i];  // reciprocal of the diagonal
+      double2 y[R];
 #pragma unroll
-          for (int s = 0; s < R; s++) v[s] = cmul(v[s], d);
-        }
-        const double2 tli = (lane > i && lane < nb) ? tb[lane][i] : make_double2(0.0, 0.0);
+      for (int s = 0; s < R; s++) y[s] = make_double2(0.0, 0.0);
+      for (int i = 0; i < nb; i++) {  // times the inverted triangle
+        const double2 tli = lane >= i && lane < nb ? tb[lane][i] : make_double2(0.0, 0.0);
 #pragma unroll
         for (int s = 0; s < R; s++) {
-          const double2 xi = make_double2(__shfl_sync(0xffffffffu, v[s].x, i),
-                                          __shfl_sync(0xffffffffu, v[s].y, i));
-          if (lane > i && lane < nb) v[s] = cfms(v[s], tli, xi);
+          const double2 xi = make_double2(-__shfl_sync(0xffffffffu, v[s].x, i),
+                                          -__shfl_sync(0xffffffffu, v[s].y, i));
+          y[s] = cfms(y[s], tli, xi);
         }
       }
+#pragma unroll
+      for (int s = 0; s < R; s++) v[s] = y[s];
       if (lane < nb)
 #pragma unroll
         for (int s = 0; s < R; s++)
@@ -842,8 +565,8 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_fwd(SolveArgs a) {
 // The right-hand-side values of the summed index pass through shared memory
 // in chunks of kThreads, so each thread's dot product streams its matrix row.
 template <int R>
-__global__ void __launch_bounds__(sp::kThreads) k_sp_solve_rect(SolveArgs a, int fwd) {
-  __shared__ double2 xc[sp::kThreads][R];
+__global__ void __launch_bounds__(kThreads) k_sp_solve_rect(SolveArgs a, int fwd) {
+  __shared__ double2 xc[kThreads][R];
   const SpFront f = a.fr[a.fronts[blockIdx.x]];
   const int r0 = blockIdx.z * R, nr = min(R, a.nrhs - r0);
   const int rows = fwd ? f.m : f.k, cols = fwd ? f.k : f.m;
@@ -900,7 +623,7 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_rect(SolveArgs a, int
 }
 
 template <int R>
-__global__ void __launch_bounds__(sp::kThreads) k_sp_solve_bwd(SolveArgs a) {
+__global__ void __launch_bounds__(kThreads) k_sp_solve_bwd(SolveArgs a) {
   __shared__ double2 xs[32][R];
   __shared__ double2 tb[32][33];  // the block's diagonal triangle, op applied
   const SpFront f = a.fr[a.fronts[blockIdx.x]];
@@ -919,7 +642,7 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_bwd(SolveArgs a) {
     for (int q = tid; q < nb * nb; q += blockDim.x) {
       const int i = q % nb, j = q / nb;
       if (i < j) tb[i][j] = sp_el(F, n, jb + i, jb + j, tr);
-      if (i == j && tr == 0) tb[i][i] = cdiv(make_double2(1.0, 0.0), sp_el(F, n, jb + i, jb + i, tr));
+      if (i == j) tb[i][i] = tr == 0 ? sp_el(F, n, jb + i, jb + i, tr) : make_double2(1.0, 0.0);
     }
     __syncthreads();
     if (warp == 0) {
@@ -927,20 +650,20 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_bwd(SolveArgs a) {
 #pragma unroll
       for (int s = 0; s < R; s++)
         v[s] = (lane < nb && s < nr) ? x[(long long)s * a.ndof + ow[jb + lane]] : make_double2(0.0, 0.0);
-      for (int i = nb - 1; i >= 0; i--) {
-        if (tr == 0 && lane == i) {
-          const double2 d = tb[i][i];  // reciprocal of the diagonal
+      double2 y[R];
 #pragma unroll
-          for (int s = 0; s < R; s++) v[s] = cmul(v[s], d);
-        }
-        const double2 tli = lane < i ? tb[lane][i] : make_double2(0.0, 0.0);
+      for (int s = 0; s < R; s++) y[s] = make_double2(0.0, 0.0);
+      for (int i = 0; i < nb; i++) {  // times the inverted triangle
+        const double2 tli = lane <= i ? tb[lane][i] : make_double2(0.0, 0.0);
 #pragma unroll
         for (int s = 0; s < R; s++) {
-          const double2 xi = make_double2(__shfl_sync(0xffffffffu, v[s].x, i),
-                                          __shfl_sync(0xffffffffu, v[s].y, i));
-          if (lane < i) v[s] = cfms(v[s], tli, xi);
+          const double2 xi = make_double2(-__shfl_sync(0xffffffffu, v[s].x, i),
+                                          -__shfl_sync(0xffffffffu, v[s].y, i));
+          y[s] = cfms(y[s], tli, xi);
         }
       }
+#pragma unroll
+      for (int s = 0; s < R; s++) v[s] = y[s];
       if (lane < nb)
 #pragma unroll
         for (int s = 0; s < R; s++)
@@ -969,7 +692,7 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_bwd(SolveArgs a) {
   if (tr != 0 && tid < nr) {  // inverse row interchanges
     double2 *xr = x + (long long)tid * a.ndof;
     for (int j = k - 1; j >= 0; j--) {
-      const int p = (int)a.piv[f.own0 + j] - 1;
+      const int p = a.swap[f.own0 + j];
       if (p != j) {
         const double2 t = xr[ow[j]];
         xr[ow[j]] = xr[ow[p]];
@@ -985,21 +708,11 @@ __global__ void __launch_bounds__(sp::kThreads) k_sp_solve_bwd(SolveArgs a) {
 void free_sparse(Ctx *c) {
   SparseLU *s = c->sparse;
   if (!s) return;
-  void *ptrs[] = {s->d_fr,      s->d_own,     s->d_bnd,     s->d_ea,      s->d_lev_fronts,
-                  s->d_ent_idx, s->d_ent_loc, s->d_fac,     s->d_piv,     s->d_work[0],
-                  s->d_work[1], s->d_info};
+  void *ptrs[] = {s->d_fr,   s->d_own,  s->d_bnd,  s->d_pull,    s->d_lev_fronts, s->d_ent_idx,
+                  s->d_ent_loc, s->d_fac, s->d_perm, s->d_swap, s->d_work[0], s->d_work[1],
+                  s->d_info};
   for (void *p : ptrs)
     if (p) cudaFree(p);
-  for (SpLane &ln : s->lane) {
-    if (ln.dwork) cudaFree(ln.dwork);
-    if (ln.d_getrf_info) cudaFree(ln.d_getrf_info);
-    if (ln.par) cusolverDnDestroyParams(ln.par);
-    if (ln.sol) cusolverDnDestroy(ln.sol);
-    if (ln.blas) cublasDestroy(ln.blas);
-    if (ln.done) cudaEventDestroy(ln.done);
-    if (ln.st) cudaStreamDestroy(ln.st);
-  }
-  if (s->level_ready) cudaEventDestroy(s->level_ready);
   delete s;
   c->sparse = nullptr;
 }
@@ -1030,28 +743,11 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
     const int r = sparse_analyse(c, s, st, msg);
     if (r) return r;
   }
-  if (!s->level_ready) {
-    SPCK(cudaFuncSetAttribute(k_sp_factor_blk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(sizeof(double2) * sp::kSmallN * sp::kNb)),
-         "kernel attributes");
-    SPCK(cudaEventCreateWithFlags(&s->level_ready, cudaEventDisableTiming), "events");
-    for (SpLane &ln : s->lane) {
-      SPCK(cudaStreamCreateWithFlags(&ln.st, cudaStreamNonBlocking), "streams");
-      SPCK(cudaEventCreateWithFlags(&ln.done, cudaEventDisableTiming), "events");
-      SPCK(cudaMalloc(&ln.d_getrf_info, sizeof(int)), "status");
-      if (cusolverDnCreate(&ln.sol) != CUSOLVER_STATUS_SUCCESS ||
-          cusolverDnCreateParams(&ln.par) != CUSOLVER_STATUS_SUCCESS ||
-          cublasCreate(&ln.blas) != CUBLAS_STATUS_SUCCESS ||
-          cusolverDnSetStream(ln.sol, ln.st) != CUSOLVER_STATUS_SUCCESS ||
-          cublasSetStream(ln.blas, ln.st) != CUBLAS_STATUS_SUCCESS) {
-        *msg = "sparse solve: cuSOLVER / cuBLAS handle creation failed";
-        return FEM25_ERR_CUDA;
-      }
-    }
-  }
+  SPCK(sparse_factor_attributes(), "kernel attributes");
   if (!s->d_fac) {
     SPCK(cudaMalloc(&s->d_fac, sizeof(double2) * std::max(s->fac_elems, 1LL)), "factor store");
-    SPCK(cudaMalloc(&s->d_piv, sizeof(int64_t) * std::max(c->ndof, 1)), "pivots");
+    SPCK(cudaMalloc(&s->d_perm, sizeof(int) * std::max(c->ndof, 1)), "pivots");
+    SPCK(cudaMalloc(&s->d_swap, sizeof(int) * std::max(c->ndof, 1)), "pivots");
     SPCK(cudaMalloc(&s->d_work[0], sizeof(double2) * std::max(s->max_work, 1LL)), "work");
     SPCK(cudaMalloc(&s->d_work[1], sizeof(double2) * std::max(s->max_work, 1LL)), "work");
     SPCK(cudaMalloc(&s->d_info, sizeof(int)), "status");
@@ -1060,96 +756,9 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
   const double2 *csr = reinterpret_cast<const double2 *>(csr128);
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-  for (int l = s->nlevel - 1; l >= 0; l--) {
-    double2 *W = s->d_work[l & 1], *Wc = s->d_work[(l + 1) & 1];
-    const int nfl = (int)s->lev[l].size();
-    const int *dfr = s->d_lev_fronts + s->lev_off[l];
-    SPCK(cudaMemsetAsync(W, 0, sizeof(double2) * s->lev_work[l], st), "work");
-    const long long ne = s->lev_ent0[l + 1] - s->lev_ent0[l];
-    if (ne > 0) {
-      const int grid = (int)std::min<long long>((ne + 255) / 256, (long long)nsm * 16);
-      k_sp_assemble<<<grid, 256, 0, st>>>(ne, s->d_ent_idx + s->lev_ent0[l],
-                                          s->d_ent_loc + s->lev_ent0[l], csr, W);
-    }
-    // more CTAs per front where the level has few fronts
-    const unsigned ysplit = (unsigned)std::max(1, std::min(64, 2 * nsm / std::max(nfl, 1)));
-    if (l + 1 < s->nlevel)
-      for (int slot = 0; slot < 2; slot++)
-        k_sp_extend_add<<<dim3(nfl, ysplit), 256, 0, st>>>(dfr, s->d_fr, s->d_ea, Wc, W, slot);
-    SPCK(cudaGetLastError(), "assembly");
-    // one CTA per front up to kSmallN rows; larger fronts: dense library calls
-    const int nsmall = s->lev_nsmall[l];
-    if (nsmall > 0) {
-      const size_t sm = sizeof(double2) * (size_t)s->lev_nmax_small[l] * sp::kNb;
-      k_sp_factor_blk<<<nsmall, sp::kFacThreads, sm, st>>>(dfr, nsmall, s->d_fr, W, s->d_piv,
-                                                         s->d_info);
-      SPCK(cudaGetLastError(), "small fronts");
-    }
-    std::vector<int> large(s->lev[l].begin() + nsmall, s->lev[l].end());
-    // the level's large fronts spread over the lanes' streams, joined back
-    // into the caller's stream before the factors are stored
-    const int nl = (int)std::min<size_t>(large.size(), sp::kLanes);
-    if (nl > 0) {
-      SPCK(cudaEventRecord(s->level_ready, st), "events");
-      for (int q = 0; q < nl; q++)
-        SPCK(cudaStreamWaitEvent(s->lane[q].st, s->level_ready, 0), "events");
-    }
-    for (size_t q = 0; q < large.size(); q++) {
-      const int t = large[q];
-      SpLane &ln = s->lane[q % sp::kLanes];
-      const SpFront &f = s->fr[t];
-      const int64_t n = (int64_t)f.k + f.m, k = f.k, m = f.m;
-      if (k == 0) continue;
-      double2 *F = W + f.work0;
-      size_t dbytes = 0, hbytes = 0;
-      if (cusolverDnXgetrf_bufferSize(ln.sol, ln.par, k, k, CUDA_C_64F, F, n, CUDA_C_64F, &dbytes,
-                                      &hbytes) != CUSOLVER_STATUS_SUCCESS) {
-        *msg = "sparse solve: getrf workspace query failed";
-        return FEM25_ERR_CUDA;
-      }
-      if (dbytes > ln.dwork_bytes) {
-        // the lane's earlier calls may still use the old workspace
-        SPCK(cudaStreamSynchronize(ln.st), "workspace");
-        if (ln.dwork) SPCK(cudaFree(ln.dwork), "workspace");
-        ln.dwork = nullptr;
-        SPCK(cudaMalloc(&ln.dwork, dbytes), "workspace");
-        ln.dwork_bytes = dbytes;
-      }
-      if (hbytes > ln.hwork.size()) ln.hwork.resize(hbytes);
-      int64_t *ipiv = s->d_piv + f.own0;
-      if (cusolverDnXgetrf(ln.sol, ln.par, k, k, CUDA_C_64F, F, n, ipiv, CUDA_C_64F, ln.dwork,
-                           dbytes, hbytes ? ln.hwork.data() : nullptr, hbytes,
-                           ln.d_getrf_info) != CUSOLVER_STATUS_SUCCESS) {
-        *msg = "sparse solve: getrf failed";
-        return FEM25_ERR_CUDA;
-      }
-      // a zero pivot of this front: recorded as the front's id in the status word
-      k_sp_getrf_status<<<1, 1, 0, ln.st>>>(ln.d_getrf_info, s->d_info, t);
-      if (m > 0) {
-        k_sp_laswp<<<(int)std::min<int64_t>((m + 127) / 128, 1024), 128, 0, ln.st>>>(
-            F, (int)n, (int)k, (int)k, (int)n, ipiv);
-        SPCK(cudaGetLastError(), "laswp");
-        const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0),
-                              mone = make_cuDoubleComplex(-1.0, 0.0);
-        cuDoubleComplex *A = reinterpret_cast<cuDoubleComplex *>(F);
-        if (cublasZtrsm(ln.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
-                        CUBLAS_DIAG_UNIT, (int)k, (int)m, &one, A, (int)n, A + k * n, (int)n) ||
-            cublasZtrsm(ln.blas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
-                        CUBLAS_DIAG_NON_UNIT, (int)m, (int)k, &one, A, (int)n, A + k, (int)n) ||
-            cublasZgemm(ln.blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)m, (int)m, (int)k, &mone, A + k,
-                        (int)n, A + k * n, (int)n, &one, A + k + k * n, (int)n)) {
-          *msg = "sparse solve: trsm / gemm failed";
-          return FEM25_ERR_CUDA;
-        }
-      }
-    }
-    for (int q = 0; q < nl; q++) {
-      SPCK(cudaEventRecord(s->lane[q].done, s->lane[q].st), "events");
-      SPCK(cudaStreamWaitEvent(st, s->lane[q].done, 0), "events");
-    }
-    k_sp_store<<<dim3(nfl, ysplit), 256, 0, st>>>(dfr, s->d_fr, W, s->d_fac);
-    SPCK(cudaGetLastError(), "factor store");
-  }
+  for (int l = s->nlevel - 1; l >= 0; l--)  // from the leaves
+    SPCK(sparse_factor_level(s, l, csr, s->d_work[l & 1], s->d_work[(l + 1) & 1], nsm, st),
+         "factorisation");
   // zero pivots of any front
   int info = 0;
   SPCK(cudaMemcpyAsync(&info, s->d_info, sizeof(int), cudaMemcpyDeviceToHost, st), "status");
@@ -1167,20 +776,20 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
 template <int R>
 static void sparse_solve_levels(const SparseLU *s, SolveArgs a, cudaStream_t st) {
   const unsigned nchunk = (unsigned)((a.nrhs + R - 1) / R);
-  auto tiles = [](int rows) { return (unsigned)std::max(1, (rows + sp::kThreads - 1) / sp::kThreads); };
+  auto tiles = [](int rows) { return (unsigned)std::max(1, (rows + kThreads - 1) / kThreads); };
   for (int l = s->nlevel - 1; l >= 0; l--) {  // forward, from the leaves
     a.fronts = s->d_lev_fronts + s->lev_off[l];
     const unsigned nfl = (unsigned)s->lev[l].size();
-    k_sp_solve_fwd<R><<<dim3(nfl, nchunk), sp::kThreads, 0, st>>>(a);
+    k_sp_solve_fwd<R><<<dim3(nfl, nchunk), kThreads, 0, st>>>(a);
     if (s->lev_mmax[l] > 0)
-      k_sp_solve_rect<R><<<dim3(nfl, tiles(s->lev_mmax[l]), nchunk), sp::kThreads, 0, st>>>(a, 1);
+      k_sp_solve_rect<R><<<dim3(nfl, tiles(s->lev_mmax[l]), nchunk), kThreads, 0, st>>>(a, 1);
   }
   for (int l = 0; l < s->nlevel; l++) {  // backward, from the root
     a.fronts = s->d_lev_fronts + s->lev_off[l];
     const unsigned nfl = (unsigned)s->lev[l].size();
     if (s->lev_mmax[l] > 0)
-      k_sp_solve_rect<R><<<dim3(nfl, tiles(s->lev_kmax[l]), nchunk), sp::kThreads, 0, st>>>(a, 0);
-    k_sp_solve_bwd<R><<<dim3(nfl, nchunk), sp::kThreads, 0, st>>>(a);
+      k_sp_solve_rect<R><<<dim3(nfl, tiles(s->lev_kmax[l]), nchunk), kThreads, 0, st>>>(a, 0);
+    k_sp_solve_bwd<R><<<dim3(nfl, nchunk), kThreads, 0, st>>>(a);
   }
 }
 
@@ -1190,12 +799,12 @@ int sparse_solve(Ctx *c, int nrhs, int trans, double *rhs, cudaStream_t st, std:
     *msg = "sparse solve: no factorisation (call fem25_sparse_factor_dev first)";
     return FEM25_ERR_ARG;
   }
-  SolveArgs a{nullptr, s->d_fr, s->d_own, s->d_bnd, s->d_fac, s->d_piv,
+  SolveArgs a{nullptr, s->d_fr, s->d_own, s->d_bnd, s->d_fac, s->d_swap,
               reinterpret_cast<double2 *>(rhs), c->ndof, nrhs, trans};
   if (nrhs == 1)
     sparse_solve_levels<1>(s, a, st);
   else
-    sparse_solve_levels<sp::kRhsPerCta>(s, a, st);
+    sparse_solve_levels<kRhsPerCta>(s, a, st);
   SPCK(cudaGetLastError(), "solve");
   return 0;
 }
