@@ -31,16 +31,12 @@
 // blocks of 32 rows whose diagonal blocks the store holds inverted.
 #include <algorithm>
 #include <cstdio>
+#include <cstdlib>
 #include <numeric>
 
 #include "sparse.cuh"
 
 namespace fem25 {
-
-namespace {
-constexpr int kThreads = 256;
-constexpr int kRhsPerCta = 8;  // right-hand sides per solve CTA
-}  // namespace
 
 // ---------------------------------------------------------------------------
 // symbolic analysis (host)
@@ -442,264 +438,533 @@ static int sparse_analyse(Ctx *c, SparseLU *s, cudaStream_t st, std::string *msg
 // ---------------------------------------------------------------------------
 // solve (device): x is [nrhs][NDOF]
 // ---------------------------------------------------------------------------
-// The triangular solves of one front, blocked by 32 rows: warp 0 solves the
-// 32 x 32 diagonal triangle of a block with the block's right-hand-side
-// values in registers (lane = row; values passed on by shuffles), the CTA
-// then updates the rows still to come with the solved block (kept in shared
-// memory): two CTA barriers per 32 rows.  Row r of the own block is the DOF
-// own[r]; the right-hand sides [r0, r0 + nr) of x (one CTA per group of
-// kRhsPerCta).
-//   op(A) = A    forward: interchanges, L11 (unit lower), x_b -= L21 x_own
-//                backward: x_own -= U12 x_b, U11 (upper)
-//   A^T / A^H    forward: U11^op (lower), x_b -= U12^op x_own
-//                backward: x_own -= L21^op x_b, L11^op (unit upper), inverse
-//                interchanges
-// The boundary rows x_b of a front belong to ancestors; fronts of one level
-// may share them, so the forward updates add with atomics.
+// Per front, with y its own rows of x and x_b its boundary rows:
+//   op(A) = A    forward: y = L11^-1 P y, x_b -= L21 y
+//                backward: y -= U12 x_b, y = U11^-1 y
+//   A^T / A^H    forward: y = U11^-op y, x_b -= U12^op y
+//                backward: y -= L21^op x_b, y = P^T L11^-op y
+// Bound: reading the factors (once a pass for a group of right-hand sides); the
+// operations are 8 flops a factor entry and right-hand side.  Every factor entry
+// is read by one lane of one warp straight into a tensor-core operand (8 rows x
+// 4 columns a warp, 128-byte column pieces, or 64-byte ones of op(A) = A^T) and
+// meets 8 NT right-hand sides from shared memory, so the factors need no staging
+// and one right-hand side is the same kernel with 7 idle columns (its padded
+// operations stay under the time of the reads).  The triangles are products with
+// the inverted 32 x 32 diagonal blocks, two barriers a block.
+// A front's boundary rows belong to ancestors and fronts of one level share
+// them, so the forward updates add with atomics.
 struct SolveArgs {
   const int *fronts;
   const SpFront *fr;
   const int *own, *bnd;
   const double2 *fac;
-  const int *swap;
+  const int *perm;
   double2 *x;
   int ndof, nrhs, trans;  // trans 0: A, 1: A^T, 2: A^H
 };
 
-__device__ __forceinline__ double2 sp_op(double2 v, int trans) {
-  return trans == 2 ? cconj(v) : v;
+// entries (r, c) of a block of op(A): p[r rs + c cs], conjugated by sg = -1
+struct SpView {
+  const double2 *p;
+  long long rs, cs;
+  double sg;
+  __device__ __forceinline__ double2 at(int r, int c) const {
+    const double2 v = __ldg(p + r * rs + c * cs);
+    return make_double2(v.x, sg * v.y);
+  }
+};
+
+// One front's step of the forward (fwd) or backward pass
+struct SpStep {
+  int k, m;
+  bool unit;        // the triangle's diagonal is 1
+  SpView tri, rect; // triangle (own x own), rectangle (fwd: boundary x own, bwd: own x boundary)
+  __device__ __forceinline__ SpStep(const SolveArgs &a, const SpFront &f, bool fwd) {
+    k = f.k;
+    m = f.m;
+    const long long n = (long long)f.k + f.m;
+    const double2 *L = a.fac + f.fac0, *U12 = L + n * f.k;
+    const bool t = a.trans != 0;
+    const double sg = a.trans == 2 ? -1.0 : 1.0;
+    unit = fwd != t;
+    tri = t ? SpView{L, n, 1, sg} : SpView{L, 1, n, sg};
+    if (fwd)
+      rect = t ? SpView{U12, f.k, 1, sg} : SpView{L + f.k, 1, n, sg};
+    else
+      rect = t ? SpView{L + f.k, n, 1, sg} : SpView{U12, 1, f.k, sg};
+  }
+  // entry of the inverted diagonal block's triangle
+  __device__ __forceinline__ double2 diag(int r, int c, bool lower) const {
+    if (r >= k || c >= k || (lower ? c > r : c < r)) return make_double2(0.0, 0.0);
+    if (r == c && unit) return make_double2(1.0, 0.0);
+    return tri.at(r, c);
+  }
+};
+
+// z[NT] (8 rows from r0 x 8 NT columns) += V(r0.., c0..c0 + nc) Y, Y in shared
+// memory with row stride 8 NT + 2 (free of conflicts for the operand's lanes) and
+// zero rows from nc to the next multiple of 4.  Rows of V end at nr: the lanes
+// past them (and past the last column) read the last one, and their rows of z
+// are not to be kept.
+template <int NT>
+__device__ __forceinline__ void sp_product(const SpView &V, int r0, int nr, int c0, int nc,
+                                           const double2 *Y, ZTile (&z)[NT]) {
+  constexpr int ld = 8 * NT + 2;
+  const int lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+  const double2 *row = V.p + (long long)min(r0 + lr, nr - 1) * V.rs + c0 * V.cs;
+  const long long cs4 = 4 * V.cs;
+  Y += lk * ld + lr;
+  for (int q0 = 0; q0 < nc; q0 += 32) {
+    double2 a[8];
+    if (q0 + 32 <= nc) {
+      const double2 *p = row + (q0 + lk) * V.cs;
+#pragma unroll
+      for (int q = 0; q < 8; q++) a[q] = __ldg(p + q * cs4);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; q++) a[q] = __ldg(row + min(q0 + 4 * q + lk, nc - 1) * V.cs);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (q0 + 4 * q < nc) {
+        const double2 v = make_double2(a[q].x, V.sg * a[q].y);
+#pragma unroll
+        for (int t = 0; t < NT; t++) z[t].mma(v, Y[(q0 + 4 * q) * ld + 8 * t]);
+      }
+  }
 }
 
-// element (i, j) of op(T) for the front's F11 (ld n) or L21 rows: op(T)(i, j)
-// = T(i, j) for A, T(j, i) (conjugated for A^H) for A^T / A^H
-__device__ __forceinline__ double2 sp_el(const double2 *T, long long n, int i, int j, int trans) {
-  return trans == 0 ? T[i + (long long)j * n] : sp_op(T[j + (long long)i * n], trans);
+// Y[r][s] = x(s0 + s, idx[pm ? pm[r] : r]), zero past n rows (up to npad) and ns
+// columns.  With 32 columns a lane keeps its rows and a warp walks columns (the
+// index is read once); with few, a warp takes 32 rows of a column at a time, so
+// that one right-hand side still spreads over the warps.
+template <int NT, int NW>
+__device__ __forceinline__ void sp_gather(const SolveArgs &a, const int *idx, const int *pm, int n,
+                                          int npad, int s0, int ns, double2 *Y) {
+  constexpr int ld = 8 * NT + 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double2 zero = make_double2(0.0, 0.0);
+  if constexpr (NT == 4) {
+    for (int r = lane; r < npad; r += 32) {
+      const int d = r < n ? idx[pm ? pm[r] : r] : -1;
+#pragma unroll 4
+      for (int s = warp; s < 8 * NT; s += NW)
+        Y[r * ld + s] = d >= 0 && s < ns ? a.x[(long long)(s0 + s) * a.ndof + d] : zero;
+    }
+  } else {
+    const int nch = (npad + 31) / 32;
+#pragma unroll 4
+    for (int it = warp; it < nch * ns; it += NW) {
+      const int ch = it / ns, s = it - ch * ns, r = 32 * ch + lane;
+      double2 v = zero;
+      if (r < n) v = a.x[(long long)(s0 + s) * a.ndof + idx[pm ? pm[r] : r]];
+      if (r < npad) Y[r * ld + s] = v;
+    }
+    if (ns < 8 * NT)
+      for (int e = threadIdx.x; e < npad * 8 * NT; e += 32 * NW)
+        if (e % (8 * NT) >= ns) Y[e / (8 * NT) * ld + e % (8 * NT)] = zero;
+  }
+}
+template <int NT, int NW>
+__device__ __forceinline__ void sp_scatter(const SolveArgs &a, const int *idx, const int *pm, int n,
+                                           int s0, int ns, const double2 *Y) {
+  constexpr int ld = 8 * NT + 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if constexpr (NT == 4) {
+    for (int r = lane; r < n; r += 32) {
+      const int d = idx[pm ? pm[r] : r];
+#pragma unroll 4
+      for (int s = warp; s < ns; s += NW) a.x[(long long)(s0 + s) * a.ndof + d] = Y[r * ld + s];
+    }
+  } else {
+    const int nch = (n + 31) / 32;
+#pragma unroll 4
+    for (int it = warp; it < nch * ns; it += NW) {
+      const int ch = it / ns, s = it - ch * ns, r = 32 * ch + lane;
+      if (r < n) a.x[(long long)(s0 + s) * a.ndof + idx[pm ? pm[r] : r]] = Y[r * ld + s];
+    }
+  }
 }
 
-template <int R>
-__global__ void __launch_bounds__(kThreads) k_sp_solve_fwd(SolveArgs a) {
-  __shared__ double2 xs[32][R];
-  __shared__ double2 tb[32][33];  // the block's diagonal triangle, op applied
-  const SpFront f = a.fr[a.fronts[blockIdx.x]];
-  const int r0 = blockIdx.y * R, nr = min(R, a.nrhs - r0);
-  if (nr <= 0 || f.k == 0) return;
-  const long long n = (long long)f.k + f.m;
-  const int k = f.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int *ow = a.own + f.own0;
-  const double2 *F = a.fac + f.fac0;          // F11 and L21, ld n
-  double2 *x = a.x + (long long)r0 * a.ndof;
-  const int tr = a.trans;
-  if (tr == 0 && tid < nr) {  // row interchanges of P
-    double2 *xr = x + (long long)tid * a.ndof;
-    for (int j = 0; j < k; j++) {
-      const int p = a.swap[f.own0 + j];
-      if (p != j) {
-        const double2 t = xr[ow[j]];
-        xr[ow[j]] = xr[ow[p]];
-        xr[ow[p]] = t;
+// rows r0 + lane / 4 of x(rows idx) -= z, by atomics or plainly
+template <int NT, bool ATOMIC>
+__device__ __forceinline__ void sp_subtract(const SolveArgs &a, const int *idx, int r0, int nr,
+                                            int s0, const ZTile (&z)[NT]) {
+  const int lane = threadIdx.x & 31, r = r0 + (lane >> 2);
+  if (r >= nr) return;
+  double2 *row = a.x + idx[r];
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int s = s0 + 8 * t + 2 * (lane & 3) + h;
+      if (s >= a.nrhs) continue;
+      double2 *o = row + (long long)s * a.ndof;
+      if (ATOMIC) {
+        atomicAdd(&o->x, -z[t].r[h]);
+        atomicAdd(&o->y, -z[t].i[h]);
+      } else {
+        *o = make_double2(o->x - z[t].r[h], o->y - z[t].i[h]);
       }
     }
+}
+
+// Triangle of a front held in Y ([kp][8 NT + 2], rows past k zero): blocks of 32
+// rows, from the top (lower) or the bottom; NW warps.
+template <int NT, int NW>
+__device__ __forceinline__ void sp_triangle(const SpStep &st, double2 *Y, bool lower) {
+  constexpr int ld = 8 * NT + 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lk = lane & 3;
+  const int kt = (st.k + 7) / 8, nblk = (st.k + 31) / 32;
+  for (int b = 0; b < nblk; b++) {
+    const int jb = 32 * (lower ? b : nblk - 1 - b), nd = min(4, kt - jb / 8);
+    // inverted diagonal block: warp = row tile
+    ZTile z[NT];
+    if (warp < nd) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const bool in = lower ? q <= 2 * warp + 1 : q >= 2 * warp && q < 2 * nd;
+        if (in) {
+          const double2 v = st.diag(jb + 8 * warp + lr, jb + 4 * q + lk, lower);
+#pragma unroll
+          for (int t = 0; t < NT; t++) z[t].mma(v, Y[(jb + 4 * q + lk) * ld + 8 * t + lr]);
+        }
+      }
+    }
+    __syncthreads();
+    if (warp < nd)
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          Y[(jb + 8 * warp + lr) * ld + 8 * t + 2 * lk + h] = make_double2(z[t].r[h], z[t].i[h]);
+    __syncthreads();
+    // rows still to come
+    const int t0 = lower ? jb / 8 + 4 : 0, t1 = lower ? kt : jb / 8;
+    for (int ti = t0 + warp; ti < t1; ti += NW) {
+      ZTile y[NT];
+      sp_product<NT>(st.tri, 8 * ti, st.k, jb, min(32, st.k - jb), Y + jb * ld, y);
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          double2 *o = Y + (8 * ti + lr) * ld + 8 * t + 2 * lk + h;
+          if (8 * ti + lr < st.k) *o = make_double2(o->x - y[t].r[h], o->y - y[t].i[h]);
+        }
+    }
+    __syncthreads();
+  }
+}
+
+constexpr int kFwdThreads = 128;  // small fronts: CTA per (front, 8 NT right-hand sides)
+// more threads where the right-hand sides fill them
+template <int NT>
+constexpr int kBwdThreads = NT == 4 ? 256 : 128;
+constexpr int kChunk = 64;          // boundary rows staged at a time in the backward pass
+
+// Fronts with k <= kSmallK, forward: own rows in shared memory.
+template <int NT>
+__global__ void __launch_bounds__(kFwdThreads) k_sp_fwd(SolveArgs a) {
+  constexpr int NW = kFwdThreads / 32;
+  extern __shared__ double2 Y[];
+  const SpFront f = a.fr[a.fronts[blockIdx.x]];
+  if (f.k == 0) return;
+  const SpStep st(a, f, true);
+  const int s0 = blockIdx.y * 8 * NT, ns = min(8 * NT, a.nrhs - s0), kp = (f.k + 7) & ~7;
+  const int *ow = a.own + f.own0, *bd = a.bnd + f.bnd0;
+  sp_gather<NT, NW>(a, ow, a.trans ? nullptr : a.perm + f.own0, f.k, kp, s0, ns, Y);
+  __syncthreads();
+  sp_triangle<NT, NW>(st, Y, true);
+  sp_scatter<NT, NW>(a, ow, nullptr, f.k, s0, ns, Y);
+  for (int r0 = 8 * (threadIdx.x >> 5); r0 < f.m; r0 += 8 * NW) {
+    ZTile z[NT];
+    sp_product<NT>(st.rect, r0, f.m, 0, f.k, Y, z);
+    sp_subtract<NT, true>(a, bd, r0, f.m, s0, z);
+  }
+}
+
+// The same, backward: boundary rows staged in chunks, then the triangle.
+template <int NT>
+__global__ void __launch_bounds__(kBwdThreads<NT>, 512 / kBwdThreads<NT>) k_sp_bwd(SolveArgs a) {
+  constexpr int ld = 8 * NT + 2, NW = kBwdThreads<NT> / 32;
+  constexpr int kMine = (sp::kSmallK / 8 + NW - 1) / NW;  // row tiles of a warp
+  extern __shared__ double2 Y[];
+  const SpFront f = a.fr[a.fronts[blockIdx.x]];
+  if (f.k == 0) return;
+  const SpStep st(a, f, false);
+  const int s0 = blockIdx.y * 8 * NT, ns = min(8 * NT, a.nrhs - s0), kp = (f.k + 7) & ~7;
+  double2 *xb = Y + kp * ld;  // [kChunk][ld]
+  const int *ow = a.own + f.own0, *bd = a.bnd + f.bnd0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lk = lane & 3;
+  sp_gather<NT, NW>(a, ow, nullptr, f.k, kp, s0, ns, Y);
+  ZTile z[kMine][NT];
+  for (int c0 = 0; c0 < f.m; c0 += kChunk) {
+    const int nc = min(kChunk, f.m - c0);
+    __syncthreads();
+    sp_gather<NT, NW>(a, bd + c0, nullptr, nc, (nc + 3) & ~3, s0, ns, xb);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kMine; q++)
+      if (8 * (warp + NW * q) < f.k)
+        sp_product<NT>(st.rect, 8 * (warp + NW * q), f.k, c0, nc, xb, z[q]);
   }
   __syncthreads();
-  // lower triangle T: L11 (unit) for A, U11^op (non-unit) for A^T / A^H
-  for (int jb = 0; jb < k; jb += 32) {
-    const int nb = min(32, k - jb);
-    for (int q = tid; q < nb * nb; q += blockDim.x) {
-      const int i = q % nb, j = q / nb;
-      if (i > j) tb[i][j] = sp_el(F, n, jb + i, jb + j, tr);
-      if (i == j) tb[i][i] = tr != 0 ? sp_el(F, n, jb + i, jb + i, tr) : make_double2(1.0, 0.0);
-    }
-    __syncthreads();
-    if (warp == 0) {
-      double2 v[R];
 #pragma unroll
-      for (int s = 0; s < R; s++)
-        v[s] = (lane < nb && s < nr) ? x[(long long)s * a.ndof + ow[jb + lane]] : make_double2(0.0, 0.0);
-      double2 y[R];
+  for (int q = 0; q < kMine; q++) {
+    const int r = 8 * (warp + NW * q) + lr;
+    if (r < f.k)
 #pragma unroll
-      for (int s = 0; s < R; s++) y[s] = make_double2(0.0, 0.0);
-      for (int i = 0; i < nb; i++) {  // times the inverted triangle
-        const double2 tli = lane >= i && lane < nb ? tb[lane][i] : make_double2(0.0, 0.0);
+      for (int t = 0; t < NT; t++)
 #pragma unroll
-        for (int s = 0; s < R; s++) {
-          const double2 xi = make_double2(-__shfl_sync(0xffffffffu, v[s].x, i),
-                                          -__shfl_sync(0xffffffffu, v[s].y, i));
-          y[s] = cfms(y[s], tli, xi);
+        for (int h = 0; h < 2; h++) {
+          double2 *o = Y + r * ld + 8 * t + 2 * lk + h;
+          *o = make_double2(o->x - z[q][t].r[h], o->y - z[q][t].i[h]);
         }
+  }
+  __syncthreads();
+  sp_triangle<NT, NW>(st, Y, false);
+  sp_scatter<NT, NW>(a, ow, a.trans ? a.perm + f.own0 : nullptr, f.k, s0, ns, Y);
+}
+
+constexpr int kTriThreads = 512;
+constexpr size_t kTriSmemMax = 200 * 1024;
+
+// Larger fronts: their triangle, a CTA per (front, gc <= 8 right-hand sides) with
+// all own rows in shared memory ([kp][ldx]), gc the most that fit.  Block by
+// block of 32 rows, left-looking: the rows' products with everything solved so
+// far are split over four groups of warps by columns (the factor's entries loaded
+// a chunk ahead, across the barriers too), summed through shared memory, then the
+// inverted diagonal block.  Right-looking in place in x each block waited
+// for a round of x loads and stores: 370 us for 720 rows, 24 blocks; this takes
+// 170 us.
+__global__ void __launch_bounds__(kTriThreads) k_sp_tri(SolveArgs a, int fwd, int gc, int ldx) {
+  extern __shared__ double2 X[];
+  __shared__ double2 part[4][32][9];
+  const SpFront f = a.fr[a.fronts[blockIdx.x]];
+  if (f.k == 0) return;
+  const SpStep st(a, f, fwd);
+  const bool lower = fwd;
+  const int s0 = blockIdx.y * gc, ns = min(gc, a.nrhs - s0), k = f.k;
+  const int *ow = a.own + f.own0, *pm = a.perm + f.own0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lk = lane & 3;
+  const int rt = warp & 3, ks = warp >> 2;  // row tile, group of columns
+  const int kp = (k + 31) & ~31, nblk = kp / 32;
+  const bool perm_in = fwd && a.trans == 0, perm_out = !fwd && a.trans != 0;
+  const double2 zero = make_double2(0.0, 0.0);
+  for (int e = tid; e < kp * gc; e += kTriThreads) {
+    const int r = e % kp, s = e / kp;
+    X[r * ldx + s] = r < k && s < ns
+                         ? a.x[(long long)(s0 + s) * a.ndof + ow[perm_in ? pm[r] : r]]
+                         : zero;
+  }
+  // Rows and columns past k read the last ones instead: such rows are not kept,
+  // such columns meet the zero rows of X.
+  const long long cs = st.tri.cs, cs4 = 4 * cs;
+  auto load = [&](double2 (&v)[8], int jb, int c) {  // 32 columns from c of the row tile
+    const double2 *row = st.tri.p + (long long)min(jb + 8 * rt + lr, k - 1) * st.tri.rs;
+    if (c + 32 <= k) {
+      const double2 *p = row + (c + lk) * cs;
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = __ldg(p + q * cs4);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = __ldg(row + min(c + 4 * q + lk, k - 1) * cs);
+    }
+  };
+  const double2 *Xl = X + lk * ldx + (lr < gc ? lr : 0);
+  auto product = [&](ZTile (&z)[2], const double2 (&v)[8], int c) {
+    const double2 *xc = Xl + c * ldx;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      double2 b = xc[4 * q * ldx];
+      if (lr >= gc) b = zero;
+      z[q & 1].mma(make_double2(v[q].x, st.tri.sg * v[q].y), b);
+    }
+  };
+  auto first = [&](int b) { return 32 * (lower ? b : nblk - 1 - b); };
+  double2 va[8], vb[8], dv[8];
+  if (ks == 0) load(dv, first(0), first(0));
+  __syncthreads();
+  for (int b = 0; b < nblk; b++) {
+    const int jb = first(b), r0 = jb + 8 * rt;
+    const int c1 = lower ? jb : kp;  // columns solved so far: [0, jb) or [jb + 32, kp)
+    int c = (lower ? 0 : jb + 32) + 32 * ks;
+    ZTile z[2];
+    while (c < c1) {  // va holds the columns from c
+      if (c + 128 < c1) load(vb, jb, c + 128);
+      product(z, va, c);
+      c += 128;
+      if (c >= c1) break;
+      if (c + 128 < c1) load(va, jb, c + 128);
+      product(z, vb, c);
+      c += 128;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      part[ks][8 * rt + lr][2 * lk + h] =
+          make_double2(z[0].r[h] + z[1].r[h], z[0].i[h] + z[1].i[h]);
+    // the next block's first columns are on their way during what follows
+    const int jn = first(b + 1), cn = (lower ? 0 : jn + 32) + 32 * ks;
+    if (b + 1 < nblk && cn < (lower ? jn : kp)) load(va, jn, cn);
+    __syncthreads();
+    if (tid < 256) {
+      const int r = tid >> 3, s = tid & 7;
+      if (s < gc && jb + r < k) {
+        double2 *o = X + (jb + r) * ldx + s;
+        double2 v = *o;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          v.x -= part[q][r][s].x;
+          v.y -= part[q][r][s].y;
+        }
+        *o = v;
       }
-#pragma unroll
-      for (int s = 0; s < R; s++) v[s] = y[s];
-      if (lane < nb)
-#pragma unroll
-        for (int s = 0; s < R; s++)
-          if (s < nr) {
-            x[(long long)s * a.ndof + ow[jb + lane]] = v[s];
-            xs[lane][s] = v[s];
-          }
     }
     __syncthreads();
-    for (int r = jb + nb + tid; r < k; r += blockDim.x) {
-      double2 acc[R];
+    if (ks == 0) {
+      ZTile y[2];
 #pragma unroll
-      for (int s = 0; s < R; s++)
-        acc[s] = s < nr ? x[(long long)s * a.ndof + ow[r]] : make_double2(0.0, 0.0);
-      for (int i = 0; i < nb; i++) {
-        const double2 t = sp_el(F, n, r, jb + i, tr);
-#pragma unroll
-        for (int s = 0; s < R; s++) acc[s] = cfms(acc[s], t, xs[i][s]);
+      for (int q = 0; q < 8; q++) {
+        const int r = 8 * rt + lr, cc = 4 * q + lk;
+        if (lower ? cc > r : cc < r) dv[q] = zero;
+        if (cc == r && st.unit) dv[q] = make_double2(1.0, 0.0);
       }
+      product(y, dv, jb);
+      if (b + 1 < nblk) load(dv, jn, jn);
+      // the first four warps have all read the block before they overwrite it
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (r0 + lr < k)
 #pragma unroll
-      for (int s = 0; s < R; s++)
-        if (s < nr) x[(long long)s * a.ndof + ow[r]] = acc[s];
+        for (int h = 0; h < 2; h++)
+          if (2 * lk + h < gc)
+            X[(r0 + lr) * ldx + 2 * lk + h] =
+                make_double2(y[0].r[h] + y[1].r[h], y[0].i[h] + y[1].i[h]);
     }
+    __syncthreads();
+  }
+  for (int e = tid; e < k * ns; e += kTriThreads) {
+    const int r = e % k, s = e / k;
+    a.x[(long long)(s0 + s) * a.ndof + ow[perm_out ? pm[r] : r]] = X[r * ldx + s];
+  }
+}
+
+// Fronts whose rows do not fit shared memory keep them in x: the permutation of P
+// (inv = 0) or P^T, a CTA per (front, right-hand side) with the old values in
+// shared memory; beyond what fits, one thread replays the interchanges.
+constexpr int kPermMax = 14000;
+__global__ void k_sp_permute(SolveArgs a, const int *__restrict__ swap, int inv) {
+  extern __shared__ double2 Y[];
+  const SpFront f = a.fr[a.fronts[blockIdx.x]];
+  const int *ow = a.own + f.own0, *pm = a.perm + f.own0, *sw = swap + f.own0;
+  for (int s = blockIdx.y; s < a.nrhs; s += gridDim.y) {
+    double2 *x = a.x + (long long)s * a.ndof;
+    if (f.k > kPermMax) {
+      if (threadIdx.x == 0)
+        for (int q = 0; q < f.k; q++) {
+          const int j = inv ? f.k - 1 - q : q;
+          const double2 v = x[ow[j]];
+          x[ow[j]] = x[ow[sw[j]]];
+          x[ow[sw[j]]] = v;
+        }
+      continue;
+    }
+    for (int r = threadIdx.x; r < f.k; r += blockDim.x) Y[r] = x[ow[r]];
+    __syncthreads();
+    for (int r = threadIdx.x; r < f.k; r += blockDim.x)
+      if (inv)
+        x[ow[pm[r]]] = Y[r];
+      else
+        x[ow[r]] = Y[pm[r]];
     __syncthreads();
   }
 }
 
-// The rectangular part of a front's solve step, spread over CTAs of
-// kThreads rows each (blockIdx.y: row tile, blockIdx.z: group of
-// right-hand sides):
-//   fwd: boundary rows   x_b -= L21 x_own (A), U12^op x_own (A^T / A^H),
-//        added with atomics (fronts of a level share boundary rows)
-//   bwd: own rows        x_own -= U12 x_b (A), L21^op x_b (A^T / A^H)
-// The right-hand-side values of the summed index pass through shared memory
-// in chunks of kThreads, so each thread's dot product streams its matrix row.
-template <int R>
-__global__ void __launch_bounds__(kThreads) k_sp_solve_rect(SolveArgs a, int fwd) {
-  __shared__ double2 xc[kThreads][R];
+// Their triangle, a CTA per (front, 8 NT right-hand sides): the block being
+// solved in shared memory, the rows still to come updated in x.
+template <int NT>
+__global__ void __launch_bounds__(kTriThreads) k_sp_tri_any(SolveArgs a, int fwd) {
+  constexpr int ld = 8 * NT + 2, NW = kTriThreads / 32;
+  __shared__ double2 Y[32 * ld];
   const SpFront f = a.fr[a.fronts[blockIdx.x]];
-  const int r0 = blockIdx.z * R, nr = min(R, a.nrhs - r0);
-  const int rows = fwd ? f.m : f.k, cols = fwd ? f.k : f.m;
-  const int row0 = blockIdx.y * blockDim.x;
-  if (nr <= 0 || row0 >= rows || cols == 0) return;
-  const long long n = (long long)f.k + f.m;
-  const int k = f.k, tid = threadIdx.x, tr = a.trans;
-  const double2 *F = a.fac + f.fac0, *U12 = F + n * k;
-  const int *rowidx = (fwd ? a.bnd + f.bnd0 : a.own + f.own0);
-  const int *colidx = (fwd ? a.own + f.own0 : a.bnd + f.bnd0);
-  double2 *x = a.x + (long long)r0 * a.ndof;
-  const int r = row0 + tid;
-  double2 acc[R];
-#pragma unroll
-  for (int s = 0; s < R; s++) acc[s] = make_double2(0.0, 0.0);
-  for (int c0 = 0; c0 < cols; c0 += blockDim.x) {
-    const int nc = min((int)blockDim.x, cols - c0);
-    __syncthreads();
-    if (tid < nc) {
-      const int d = colidx[c0 + tid];
-#pragma unroll
-      for (int s = 0; s < R; s++)
-        xc[tid][s] = s < nr ? x[(long long)s * a.ndof + d] : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    if (r < rows) {
-#pragma unroll 4
-      for (int j = 0; j < nc; j++) {
-        const int c = c0 + j;
-        // element (r, c) of the rectangular block
-        double2 t;
-        if (fwd)
-          t = tr == 0 ? F[k + r + (long long)c * n] : sp_op(U12[c + (long long)r * k], tr);
-        else
-          t = tr == 0 ? U12[r + (long long)c * k] : sp_op(F[k + c + (long long)r * n], tr);
-#pragma unroll
-        for (int s = 0; s < R; s++) acc[s] = cfms(acc[s], t, xc[j][s]);
-      }
-    }
-  }
-  if (r >= rows) return;
-  const int d = rowidx[r];
-#pragma unroll
-  for (int s = 0; s < R; s++)
-    if (s < nr) {
-      double2 *o = x + (long long)s * a.ndof + d;
-      if (fwd) {  // acc = -(product)
-        atomicAdd(reinterpret_cast<double *>(o), acc[s].x);
-        atomicAdd(reinterpret_cast<double *>(o) + 1, acc[s].y);
-      } else {
-        *o = make_double2(o->x + acc[s].x, o->y + acc[s].y);
-      }
-    }
-}
-
-template <int R>
-__global__ void __launch_bounds__(kThreads) k_sp_solve_bwd(SolveArgs a) {
-  __shared__ double2 xs[32][R];
-  __shared__ double2 tb[32][33];  // the block's diagonal triangle, op applied
-  const SpFront f = a.fr[a.fronts[blockIdx.x]];
-  const int r0 = blockIdx.y * R, nr = min(R, a.nrhs - r0);
-  if (nr <= 0 || f.k == 0) return;
-  const long long n = (long long)f.k + f.m;
-  const int k = f.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const SpStep st(a, f, fwd);
+  const bool lower = fwd;
+  const int s0 = blockIdx.y * 8 * NT, ns = min(8 * NT, a.nrhs - s0), k = f.k;
   const int *ow = a.own + f.own0;
-  const double2 *F = a.fac + f.fac0;
-  double2 *x = a.x + (long long)r0 * a.ndof;
-  const int tr = a.trans;
-  // upper triangle T: U11 (non-unit) for A, L11^op (unit) for A^T / A^H;
-  // blocks of 32 rows from the bottom
-  for (int jb = ((k - 1) / 32) * 32; jb >= 0; jb -= 32) {
-    const int nb = min(32, k - jb);
-    for (int q = tid; q < nb * nb; q += blockDim.x) {
-      const int i = q % nb, j = q / nb;
-      if (i < j) tb[i][j] = sp_el(F, n, jb + i, jb + j, tr);
-      if (i == j) tb[i][i] = tr == 0 ? sp_el(F, n, jb + i, jb + i, tr) : make_double2(1.0, 0.0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lk = lane & 3;
+  const int kt = (k + 7) / 8, nblk = (k + 31) / 32;
+  for (int b = 0; b < nblk; b++) {
+    const int jb = 32 * (lower ? b : nblk - 1 - b), nd = min(4, kt - jb / 8);
+    for (int e = tid; e < 32 * 8 * NT; e += kTriThreads) {
+      const int r = e % 32, s = e / 32;
+      double2 v = make_double2(0.0, 0.0);
+      if (jb + r < k && s < ns) v = a.x[(long long)(s0 + s) * a.ndof + ow[jb + r]];
+      Y[r * ld + s] = v;
     }
     __syncthreads();
-    if (warp == 0) {
-      double2 v[R];
+    ZTile z[NT];
+    if (warp < nd) {
 #pragma unroll
-      for (int s = 0; s < R; s++)
-        v[s] = (lane < nb && s < nr) ? x[(long long)s * a.ndof + ow[jb + lane]] : make_double2(0.0, 0.0);
-      double2 y[R];
+      for (int q = 0; q < 8; q++) {
+        const bool in = lower ? q <= 2 * warp + 1 : q >= 2 * warp && q < 2 * nd;
+        if (in) {
+          const double2 v = st.diag(jb + 8 * warp + lr, jb + 4 * q + lk, lower);
 #pragma unroll
-      for (int s = 0; s < R; s++) y[s] = make_double2(0.0, 0.0);
-      for (int i = 0; i < nb; i++) {  // times the inverted triangle
-        const double2 tli = lane <= i ? tb[lane][i] : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int s = 0; s < R; s++) {
-          const double2 xi = make_double2(-__shfl_sync(0xffffffffu, v[s].x, i),
-                                          -__shfl_sync(0xffffffffu, v[s].y, i));
-          y[s] = cfms(y[s], tli, xi);
+          for (int t = 0; t < NT; t++) z[t].mma(v, Y[(4 * q + lk) * ld + 8 * t + lr]);
         }
       }
-#pragma unroll
-      for (int s = 0; s < R; s++) v[s] = y[s];
-      if (lane < nb)
-#pragma unroll
-        for (int s = 0; s < R; s++)
-          if (s < nr) {
-            x[(long long)s * a.ndof + ow[jb + lane]] = v[s];
-            xs[lane][s] = v[s];
-          }
     }
     __syncthreads();
-    for (int r = tid; r < jb; r += blockDim.x) {
-      double2 acc[R];
+    if (warp < nd) {
+      const int r = jb + 8 * warp + lr;
 #pragma unroll
-      for (int s = 0; s < R; s++)
-        acc[s] = s < nr ? x[(long long)s * a.ndof + ow[r]] : make_double2(0.0, 0.0);
-      for (int i = 0; i < nb; i++) {
-        const double2 t = sp_el(F, n, r, jb + i, tr);
+      for (int t = 0; t < NT; t++)
 #pragma unroll
-        for (int s = 0; s < R; s++) acc[s] = cfms(acc[s], t, xs[i][s]);
-      }
-#pragma unroll
-      for (int s = 0; s < R; s++)
-        if (s < nr) x[(long long)s * a.ndof + ow[r]] = acc[s];
+        for (int h = 0; h < 2; h++) {
+          const int s = 8 * t + 2 * lk + h;
+          const double2 v = make_double2(z[t].r[h], z[t].i[h]);
+          Y[(8 * warp + lr) * ld + s] = v;
+          if (r < k && s < ns) a.x[(long long)(s0 + s) * a.ndof + ow[r]] = v;
+        }
+    }
+    __syncthreads();
+    const int t0 = lower ? jb / 8 + 4 : 0, t1 = lower ? kt : jb / 8;
+    for (int ti = t0 + warp; ti < t1; ti += NW) {
+      ZTile y[NT];
+      sp_product<NT>(st.tri, 8 * ti, k, jb, min(32, k - jb), Y, y);
+      sp_subtract<NT, false>(a, ow, 8 * ti, k, s0, y);
     }
     __syncthreads();
   }
-  if (tr != 0 && tid < nr) {  // inverse row interchanges
-    double2 *xr = x + (long long)tid * a.ndof;
-    for (int j = k - 1; j >= 0; j--) {
-      const int p = a.swap[f.own0 + j];
-      if (p != j) {
-        const double2 t = xr[ow[j]];
-        xr[ow[j]] = xr[ow[p]];
-        xr[ow[p]] = t;
-      }
-    }
+}
+
+// Their rectangle, 64 rows a CTA over blockIdx.y (a warp per 8), the right-hand
+// side of the summed index staged in chunks: forward x_b -= rect y (atomics),
+// backward y -= rect x_b.
+template <int NT>
+__global__ void __launch_bounds__(256) k_sp_rect(SolveArgs a, int fwd) {
+  constexpr int ld = 8 * NT + 2;
+  __shared__ double2 Y[kChunk * ld];
+  const SpFront f = a.fr[a.fronts[blockIdx.x]];
+  const SpStep st(a, f, fwd);
+  const int rows = fwd ? f.m : f.k, cols = fwd ? f.k : f.m;
+  if (64 * (int)blockIdx.y >= rows || cols == 0) return;
+  const int *ri = fwd ? a.bnd + f.bnd0 : a.own + f.own0;
+  const int *ci = fwd ? a.own + f.own0 : a.bnd + f.bnd0;
+  const int s0 = blockIdx.z * 8 * NT, ns = min(8 * NT, a.nrhs - s0);
+  const int tid = threadIdx.x, r0 = 64 * blockIdx.y + 8 * (tid >> 5);
+  ZTile z[NT];
+  for (int c0 = 0; c0 < cols; c0 += kChunk) {
+    const int nc = min(kChunk, cols - c0);
+    __syncthreads();
+    sp_gather<NT, 8>(a, ci + c0, nullptr, nc, (nc + 3) & ~3, s0, ns, Y);
+    __syncthreads();
+    if (r0 < rows) sp_product<NT>(st.rect, r0, rows, c0, nc, Y, z);
   }
+  if (r0 >= rows) return;
+  if (fwd)
+    sp_subtract<NT, true>(a, ri, r0, rows, s0, z);
+  else
+    sp_subtract<NT, false>(a, ri, r0, rows, s0, z);
 }
 
 // ---------------------------------------------------------------------------
@@ -735,6 +1000,16 @@ void sparse_info(const Ctx *c, long long *out) {
     }                                                                      \
   } while (0)
 
+template <int NT>
+static cudaError_t sparse_solve_attributes() {
+  constexpr size_t row = sizeof(double2) * (8 * NT + 2);
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_sp_fwd<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(row * sp::kSmallK));
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_sp_bwd<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(row * (sp::kSmallK + kChunk)));
+}
+
 int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *msg) {
   if (!c->sparse) c->sparse = new SparseLU();
   SparseLU *s = c->sparse;
@@ -744,6 +1019,15 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
     if (r) return r;
   }
   SPCK(sparse_factor_attributes(), "kernel attributes");
+  SPCK(cudaFuncSetAttribute(k_sp_permute, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)(sizeof(double2) * kPermMax)),
+       "kernel attributes");
+  SPCK(cudaFuncSetAttribute(k_sp_tri, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)kTriSmemMax),
+       "kernel attributes");
+  SPCK(sparse_solve_attributes<1>(), "kernel attributes");
+  SPCK(sparse_solve_attributes<2>(), "kernel attributes");
+  SPCK(sparse_solve_attributes<4>(), "kernel attributes");
   if (!s->d_fac) {
     SPCK(cudaMalloc(&s->d_fac, sizeof(double2) * std::max(s->fac_elems, 1LL)), "factor store");
     SPCK(cudaMalloc(&s->d_perm, sizeof(int) * std::max(c->ndof, 1)), "pivots");
@@ -772,25 +1056,48 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
   return 0;
 }
 
-// the level-by-level launches of one solve, R right-hand sides per CTA
-template <int R>
-static void sparse_solve_levels(const SparseLU *s, SolveArgs a, cudaStream_t st) {
-  const unsigned nchunk = (unsigned)((a.nrhs + R - 1) / R);
-  auto tiles = [](int rows) { return (unsigned)std::max(1, (rows + kThreads - 1) / kThreads); };
-  for (int l = s->nlevel - 1; l >= 0; l--) {  // forward, from the leaves
-    a.fronts = s->d_lev_fronts + s->lev_off[l];
-    const unsigned nfl = (unsigned)s->lev[l].size();
-    k_sp_solve_fwd<R><<<dim3(nfl, nchunk), kThreads, 0, st>>>(a);
-    if (s->lev_mmax[l] > 0)
-      k_sp_solve_rect<R><<<dim3(nfl, tiles(s->lev_mmax[l]), nchunk), kThreads, 0, st>>>(a, 1);
+// One level's launches of a pass, 8 NT right-hand sides a CTA
+template <int NT>
+static cudaError_t sparse_solve_level(const SparseLU *s, SolveArgs a, int l, bool fwd,
+                                      cudaStream_t st) {
+  const unsigned groups = (unsigned)((a.nrhs + 8 * NT - 1) / (8 * NT));
+  const int nsmall = s->lev_nsmall[l], nbig = (int)s->lev[l].size() - nsmall;
+  constexpr size_t row = sizeof(double2) * (8 * NT + 2);
+  a.fronts = s->d_lev_fronts + s->lev_off[l];
+  if (nsmall > 0 && s->lev_ksmall[l] > 0) {
+    const size_t kp = (size_t)(s->lev_ksmall[l] + 7) & ~7;
+    if (fwd)
+      k_sp_fwd<NT><<<dim3(nsmall, groups), kFwdThreads, row * kp, st>>>(a);
+    else
+      k_sp_bwd<NT><<<dim3(nsmall, groups), kBwdThreads<NT>, row * (kp + kChunk), st>>>(a);
   }
-  for (int l = 0; l < s->nlevel; l++) {  // backward, from the root
-    a.fronts = s->d_lev_fronts + s->lev_off[l];
-    const unsigned nfl = (unsigned)s->lev[l].size();
-    if (s->lev_mmax[l] > 0)
-      k_sp_solve_rect<R><<<dim3(nfl, tiles(s->lev_kmax[l]), nchunk), kThreads, 0, st>>>(a, 0);
-    k_sp_solve_bwd<R><<<dim3(nfl, nchunk), kThreads, 0, st>>>(a);
+  if (nbig > 0) {
+    a.fronts += nsmall;
+    const int kmax = s->lev_kmax[l], mmax = s->lev_mmax[l];
+    const dim3 rect(nbig, ((fwd ? mmax : kmax) + 63) / 64, groups);
+    // right-hand sides of a triangle's CTA: 8, or fewer so that the largest
+    // front's rows fit (strides without bank conflicts); FEM25_PANEL_WIDTH=1
+    // selects the any-size kernels, as in the factorisation
+    const size_t kp = (size_t)(kmax + 31) & ~31;
+    int gc = 8;
+    auto ldx = [](int g) { return g > 2 ? g + 2 : g; };
+    while (gc > 1 && (a.nrhs <= gc / 2 || sizeof(double2) * kp * ldx(gc) > kTriSmemMax)) gc /= 2;
+    const char *env = std::getenv("FEM25_PANEL_WIDTH");
+    const bool any = sizeof(double2) * kp * ldx(gc) > kTriSmemMax || (env && std::atoi(env) == 1);
+    const dim3 perm(nbig, std::min(a.nrhs, 65535));
+    const size_t psm = sizeof(double2) * (size_t)std::min(kmax, kPermMax);
+    if (!fwd && mmax > 0) k_sp_rect<NT><<<rect, 256, 0, st>>>(a, 0);
+    if (any) {
+      if (fwd && a.trans == 0) k_sp_permute<<<perm, 256, psm, st>>>(a, s->d_swap, 0);
+      k_sp_tri_any<NT><<<dim3(nbig, groups), kTriThreads, 0, st>>>(a, fwd);
+      if (!fwd && a.trans != 0) k_sp_permute<<<perm, 256, psm, st>>>(a, s->d_swap, 1);
+    } else {
+      k_sp_tri<<<dim3(nbig, (a.nrhs + gc - 1) / gc), kTriThreads, sizeof(double2) * kp * ldx(gc),
+                 st>>>(a, fwd, gc, ldx(gc));
+    }
+    if (fwd && mmax > 0) k_sp_rect<NT><<<rect, 256, 0, st>>>(a, 1);
   }
+  return cudaGetLastError();
 }
 
 int sparse_solve(Ctx *c, int nrhs, int trans, double *rhs, cudaStream_t st, std::string *msg) {
@@ -799,12 +1106,25 @@ int sparse_solve(Ctx *c, int nrhs, int trans, double *rhs, cudaStream_t st, std:
     *msg = "sparse solve: no factorisation (call fem25_sparse_factor_dev first)";
     return FEM25_ERR_ARG;
   }
-  SolveArgs a{nullptr, s->d_fr, s->d_own, s->d_bnd, s->d_fac, s->d_swap,
+  SolveArgs a{nullptr, s->d_fr, s->d_own, s->d_bnd, s->d_fac, s->d_perm,
               reinterpret_cast<double2 *>(rhs), c->ndof, nrhs, trans};
-  if (nrhs == 1)
-    sparse_solve_levels<1>(s, a, st);
-  else
-    sparse_solve_levels<kRhsPerCta>(s, a, st);
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+  // Right-hand sides a CTA: as many as there are, up to 32, so that the factors
+  // are read once; fewer where a level has too few fronts to fill the GPU.
+  const int most = nrhs <= 8 ? 1 : nrhs <= 16 ? 2 : 4;
+  for (int pass = 0; pass < 2; pass++)
+    for (int q = 0; q < s->nlevel; q++) {
+      const bool fwd = pass == 0;
+      const int l = fwd ? s->nlevel - 1 - q : q;  // forward from the leaves, back from the root
+      const long long nf = (long long)s->lev[l].size();
+      int nt = most;
+      while (nt > 1 && nf * ((nrhs + 8 * nt - 1) / (8 * nt)) < 2 * nsm) nt /= 2;
+      SPCK(nt == 1   ? sparse_solve_level<1>(s, a, l, fwd, st)
+           : nt == 2 ? sparse_solve_level<2>(s, a, l, fwd, st)
+                     : sparse_solve_level<4>(s, a, l, fwd, st),
+           "solve");
+    }
   SPCK(cudaGetLastError(), "solve");
   return 0;
 }
