@@ -190,6 +190,10 @@ struct Ctx {
   // fem25_cfmat_adjgrad): 3 COMPLEX*8 [NDOF] vectors and GRADL
   float2 *d_hvec = nullptr;
   float *d_hgrad = nullptr;
+  // device block of the host-array calls fem25_misfit_dev / fem25_postsolve_dev,
+  // which return after their stream is done; grown to the largest call
+  char *d_call = nullptr;
+  size_t d_call_bytes = 0;
   // misfit options (fem25_misfit_options); the defaults of the reference
   MisfitOpts mopt{2, 3, 0, 0.0f, 0.0f, 0.0f, 0.0f, 0.0, {1.0f, 0.0f}};
   // optional CUDA-event timing of the dominant kernels
