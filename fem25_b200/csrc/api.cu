@@ -88,7 +88,7 @@ int check_mesh(const fem25_mesh *m, std::string *msg) {
 }
 
 void free_ctx(Ctx *c) {
-  void *ptrs[] = {c->dt.xigll, c->dt.wts, c->dt.shl, c->dt.sf, c->dt.dsf, c->d_ieng, c->d_cdomain,
+  void *ptrs[] = {c->dt.xigll, c->dt.wts, c->dt.shl, c->dt.shn, c->dt.sf, c->dt.dsf, c->d_ieng, c->d_cdomain,
                   c->d_x, c->d_z, c->d_xd, c->d_zd, c->d_lam, c->d_mu, c->d_rho, c->d_lm,
                   c->d_irptr, c->d_jcptr, c->d_cnp, c->d_elemmat, c->d_gptr, c->d_glist, c->d_err,
                   c->d_brptr, c->d_brow, c->d_basis, c->d_ebasis, c->d_bgptr, c->d_bglist,
@@ -98,14 +98,18 @@ void free_ctx(Ctx *c) {
                   c->d_cadj_dptr, c->d_cadj_dent, c->d_cadj_w, c->d_nonpml, c->d_cdist, c->d_prim, c->d_desc,
                   c->d_tc_tab, c->d_qp, c->d_qs, c->d_cov, c->d_cov_ops, c->d_cov_opptr,
                   c->d_cov_tx, c->d_cov_node, c->d_cov_exps, c->d_maskg, c->d_avg_work, c->d_post_mrdof,
-                  c->d_post_bits, c->d_hvec, c->d_hgrad, c->d_call};
+                  c->d_post_bits, c->d_hvec, c->d_hgrad, c->d_call, c->d_tasks, c->d_tasks_pml};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &e : c->ev)
     if (e) cudaEventDestroy(e);
   for (auto &e : c->drv_ev)
     if (e) cudaEventDestroy(e);
+  for (auto &e : c->drv_elem_ev)
+    if (e) cudaEventDestroy(e);
   if (c->copy_st) cudaStreamDestroy(c->copy_st);
+  for (auto &s : c->elem_st)
+    if (s) cudaStreamDestroy(s);
   free_dense(c);
   free_sparse(c);
 }
@@ -263,6 +267,10 @@ int ensure_driver_plan(Ctx *c) {
     return fail(c, FEM25_ERR_PATTERN, "asmble_driver: DOF outside every element");
   c->drv_ev.assign(nch, nullptr);
   for (auto &e : c->drv_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+  c->drv_elem_ev.assign(nch + 1, nullptr);
+  for (auto &e : c->drv_elem_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+  for (auto &s : c->elem_st)
+    CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "element streams");
   CK(cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking), "copy stream");
   return FEM25_OK;
 }
@@ -476,6 +484,9 @@ int fem25_create(const fem25_mesh *m, int ndof, long long nzero, const int *lm, 
     CK(dalloc_copy(&c->dt.xigll, c->tab.xigll, kNint), "tables");
     CK(dalloc_copy(&c->dt.wts, c->tab.wts, kNint), "tables");
     CK(dalloc_copy(&c->dt.shl, c->tab.shl, 3 * kNen * kNq), "tables");
+    std::vector<double> shn(kNen * kNq);
+    for (int i = 0; i < kNen * kNq; i++) shn[i] = c->tab.shl[3 * i + 2];
+    CK(dalloc_copy(&c->dt.shn, shn.data(), shn.size()), "tables");
     CK(dalloc_copy(&c->dt.sf, &c->tab.sf[0][0], 4 * kNq), "tables");
     CK(dalloc_copy(&c->dt.dsf, &c->tab.dsf[0][0][0], 8 * kNq), "tables");
     CK(dalloc_copy(&c->d_ieng, reinterpret_cast<const int4 *>(m->ieng), m->nelem), "mesh");
@@ -504,6 +515,19 @@ int fem25_create(const fem25_mesh *m, int ndof, long long nzero, const int *lm, 
       if (m->cdomain[e] != 'A') nonpml.push_back(e);
     c->n_nonpml = (int)nonpml.size();
     CK(dalloc_copy(&c->d_nonpml, nonpml.data(), nonpml.size()), "element lists");
+    std::vector<int> tasks, tasks_pml;
+    c->h_task0.assign(m->nelem + 1, 0);
+    for (int e = 0; e < m->nelem; e++) {
+      const bool pml = m->cdomain[e] == 'A';
+      for (int p = 0; p < (pml ? 2 : 1); p++) {
+        tasks.push_back(2 * e + p);
+        if (pml) tasks_pml.push_back(2 * e + p);
+      }
+      c->h_task0[e + 1] = (int)tasks.size();
+    }
+    for (int e : nonpml) tasks_pml.push_back(2 * e);
+    CK(dalloc_copy(&c->d_tasks, tasks.data(), tasks.size()), "element lists");
+    CK(dalloc_copy(&c->d_tasks_pml, tasks_pml.data(), tasks_pml.size()), "element lists");
     c->mv.nelem = m->nelem;
     c->mv.nnpg = m->nnpg;
     c->mv.ieng = c->d_ieng;
@@ -595,13 +619,21 @@ int fem25_asmble_driver(fem25_ctx *h, int nzloc, char cftype, double freq, doubl
   if (r) return r;
   // every chunk's element matrices and gather are enqueued first, then the
   // host copies follow the chunks as they complete (a pageable destination
-  // makes each copy synchronous for the host, the GPU keeps computing)
-  cudaStream_t st = nullptr;
+  // makes each copy synchronous for the host, the GPU keeps computing).  The
+  // chunks alternate between two streams, so that one's last elements (a PML
+  // element takes 2.5 times as long) do not idle the GPU; a chunk's gather waits
+  // for the chunk before it too, whose own order covers the earlier ones.
   const int nch = (int)c->drv_elem.size() - 1;
+  // what the caller and earlier calls left on the default stream comes first
+  CK(cudaEventRecord(c->drv_elem_ev[nch], nullptr), "event");
+  for (cudaStream_t s : c->elem_st) CK(cudaStreamWaitEvent(s, c->drv_elem_ev[nch], 0), "event");
   for (int k = 0; k < nch; k++) {
     const long long nz0 = c->h_irptr[c->drv_row[k]] - 1, nz1 = c->h_irptr[c->drv_row[k + 1]] - 1;
+    cudaStream_t st = c->elem_st[k & 1];
     CK(launch_elem_plain(c, cftype, freq, py, c->drv_elem[k], c->drv_elem[k + 1], st),
        "element kernel");
+    CK(cudaEventRecord(c->drv_elem_ev[k], st), "event");
+    if (k > 0) CK(cudaStreamWaitEvent(st, c->drv_elem_ev[k - 1], 0), "event");
     CK(launch_gather_plain(c, nullptr, (float *)c->d_cdist, nz0, nz1, st), "gather kernel");
     CK(cudaEventRecord(c->drv_ev[k], st), "event");
   }
@@ -614,6 +646,8 @@ int fem25_asmble_driver(fem25_ctx *h, int nzloc, char cftype, double freq, doubl
        "cdist copy");
   }
   CK(cudaStreamSynchronize(c->copy_st), "cdist copy");
+  // a last chunk without rows of its own has no copy behind it
+  for (cudaStream_t s : c->elem_st) CK(cudaStreamSynchronize(s), "element streams");
   return read_err_word(c, 0);
 }
 

@@ -17,6 +17,7 @@ struct DevTables {
   double *xigll;  // [13]
   double *wts;    // [13]
   double *shl;    // [169][25][3]  SHL(3,NEN,NINT,NINT)
+  double *shn;    // [169][25]  the shape functions alone, SHL(3,:,:,:)
   double *sf;     // [169][4]
   double *dsf;    // [169][2][4]
 };
@@ -113,6 +114,10 @@ struct Ctx {
   int *d_gptr = nullptr;         // [nzero+1]
   int *d_glist = nullptr;        // contribution ids, element order per nonzero
   long long ncontrib = 0;
+  // element kernel tasks 2 element + part (two parts per PML element): in element
+  // order with h_task0[e] the first of element e, and with the PML elements first
+  int *d_tasks = nullptr, *d_tasks_pml = nullptr;
+  std::vector<int> h_task0;
   int *d_err = nullptr;          // device error word
   // batched path
   BlockCSR bcsr;
@@ -171,8 +176,8 @@ struct Ctx {
   // host on copy_st while the next chunk computes
   float2 *d_cdist = nullptr;
   std::vector<int> drv_elem, drv_row;
-  cudaStream_t copy_st = nullptr;
-  std::vector<cudaEvent_t> drv_ev;
+  cudaStream_t copy_st = nullptr, elem_st[2] = {nullptr, nullptr};
+  std::vector<cudaEvent_t> drv_ev, drv_elem_ev;
   DenseLU *dense = nullptr;
   SparseLU *sparse = nullptr;
   // fem25_assemble_dev with the FMA build of the element kernels

@@ -248,11 +248,9 @@ __device__ __forceinline__ void cmdamp_pair(const double *qc, const double *shx,
   out[8] = make_double2(me2 + ce[8].re, ce[8].im);
 }
 
-// kDisp: dispersive media (KMDAMP / CMDAMP); a separate instance so that the
-// non-dispersive kernel keeps its own register allocation
-template <bool kDisp>
+// Dispersive media (KMDAMP / CMDAMP): one node pair a thread
 __global__ void __launch_bounds__(kPlainThreads, 1)
-    k_elem_plain(MeshView mv, DevTables dt, PlainArgs pa, double2 *__restrict__ elemmat,
+    k_elem_disp(MeshView mv, DevTables dt, PlainArgs pa, double2 *__restrict__ elemmat,
                  int *__restrict__ err) {
   extern __shared__ double sm[];
   double *shx = sm + kSmShx, *shz = sm + kSmShz, *shn = sm + kSmShn, *qc = sm + kSmQ;
@@ -269,67 +267,41 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
     double *c = qc + kNqc * q;
     c[0] = g.dxdxi; c[1] = g.dxdeta; c[2] = g.dzdxi; c[3] = g.dzdeta; c[4] = g.rjac;
     double weight = dt.wts[intx] * dt.wts[intz] * g.rjac;
-    double lambda = g.lam * weight, mu = g.mu * weight, rhow = g.rho * weight;
-    if constexpr (kDisp) {
-      // KMDAMP / CMDAMP point terms (estiff25.f:592-607, 822-838)
-      double vp, vs, qpp, qss;
-      quad_qual(mv, dt, ie, q, vp, vs, qpp, qss);
-      const dcx zv = vcmplx(pa, vp, qpp), zs = vcmplx(pa, vs, qss);
-      dcx zvp2 = zmul(zv, zv), zvs2 = zmul(zs, zs);
-      double rvp2, qvp2, rvs2, qvs2;
-      if (!pml) {
-        rvp2 = zvp2.re * weight;
-        qvp2 = zvp2.im * weight;
-        rvs2 = zvs2.re * weight;
-        qvs2 = zvs2.im * weight;
-      } else {
-        zvp2 = zmul(zvp2, dcx{weight, 0.0});
-        zvs2 = zmul(zvs2, dcx{weight, 0.0});
-        rvp2 = zvp2.re;
-        qvp2 = zvp2.im;
-        rvs2 = zvs2.re;
-        qvs2 = zvs2.im;
-      }
-      c[5] = rvp2; c[6] = qvp2; c[7] = rvs2; c[8] = qvs2;
-      c[9] = -(pa.w2 * weight) + pa.w2 * pa.py2 * rvs2;   // RMCOEFF1
-      c[10] = pa.w2 * pa.py2 * qvs2;                      // QMCOEFF1
-      c[11] = -(pa.w2 * weight) + pa.w2 * pa.py2 * rvp2;  // RMCOEFF2
-      c[12] = pa.w2 * pa.py2 * qvp2;                      // QMCOEFF2
-      if (pml) {
-        // CJCM_QUAL: the damping profile uses the interpolated Vp
-        dcx ex = dcx{1.0, 0.0}, ez = dcx{1.0, 0.0};
-        if (g.xdep > 2.22e-16)
-          ex = zdampfn(g.xdep, vp, pa.pml.xwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
-                       pa.pml.fcent, pa.omega);
-        if (g.zdep > 2.22e-16)
-          ez = zdampfn(g.zdep, vp, pa.pml.zwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
-                       pa.pml.fcent, pa.omega);
-        c[13] = ex.re; c[14] = ex.im;
-        c[15] = ez.re; c[16] = ez.im;
-      }
-    } else if (!pml) {
-      double c11 = lambda + 2.0 * mu;
-      c[5] = lambda;
-      c[6] = mu;
-      c[7] = c11;
-      c[8] = -pa.w2 * (rhow - pa.py2 * mu);   // COEFFM1 (C66)
-      c[9] = -pa.w2 * (rhow - pa.py2 * c11);  // COEFFM2 (C22)
-      c[10] = pa.wpy * lambda;                // WPY*C12 = WPY*C23
-      c[11] = pa.wpy * mu;                    // WPY*C66 = WPY*C44
+    // KMDAMP / CMDAMP point terms (estiff25.f:592-607, 822-838)
+    double vp, vs, qpp, qss;
+    quad_qual(mv, dt, ie, q, vp, vs, qpp, qss);
+    const dcx zv = vcmplx(pa, vp, qpp), zs = vcmplx(pa, vs, qss);
+    dcx zvp2 = zmul(zv, zv), zvs2 = zmul(zs, zs);
+    double rvp2, qvp2, rvs2, qvs2;
+    if (!pml) {
+      rvp2 = zvp2.re * weight;
+      qvp2 = zvp2.im * weight;
+      rvs2 = zvs2.re * weight;
+      qvs2 = zvs2.im * weight;
     } else {
+      zvp2 = zmul(zvp2, dcx{weight, 0.0});
+      zvs2 = zmul(zvs2, dcx{weight, 0.0});
+      rvp2 = zvp2.re;
+      qvp2 = zvp2.im;
+      rvs2 = zvs2.re;
+      qvs2 = zvs2.im;
+    }
+    c[5] = rvp2; c[6] = qvp2; c[7] = rvs2; c[8] = qvs2;
+    c[9] = -(pa.w2 * weight) + pa.w2 * pa.py2 * rvs2;   // RMCOEFF1
+    c[10] = pa.w2 * pa.py2 * qvs2;                      // QMCOEFF1
+    c[11] = -(pa.w2 * weight) + pa.w2 * pa.py2 * rvp2;  // RMCOEFF2
+    c[12] = pa.w2 * pa.py2 * qvp2;                      // QMCOEFF2
+    if (pml) {
+      // CJCM_QUAL: the damping profile uses the interpolated Vp
       dcx ex = dcx{1.0, 0.0}, ez = dcx{1.0, 0.0};
       if (g.xdep > 2.22e-16)
-        ex = zdampfn(g.xdep, g.vel, pa.pml.xwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
+        ex = zdampfn(g.xdep, vp, pa.pml.xwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
                      pa.pml.fcent, pa.omega);
       if (g.zdep > 2.22e-16)
-        ez = zdampfn(g.zdep, g.vel, pa.pml.zwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
+        ez = zdampfn(g.zdep, vp, pa.pml.zwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
                      pa.pml.fcent, pa.omega);
-      c[5] = lambda;
-      c[6] = mu;
-      c[7] = -pa.w2 * (rhow - pa.py2 * mu);                  // COEFFM1
-      c[8] = -pa.w2 * (rhow - pa.py2 * (lambda + 2.0 * mu)); // COEFFM2
-      c[9] = ex.re; c[10] = ex.im;
-      c[11] = ez.re; c[12] = ez.im;
+      c[13] = ex.re; c[14] = ex.im;
+      c[15] = ez.re; c[16] = ez.im;
     }
   }
   __syncthreads();
@@ -347,137 +319,223 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
   if (t >= kNab) return;
   const int a = t / kNen, b = t % kNen;
   double2 *out = elemmat + ((size_t)e * kNab + t) * 9;
-  if constexpr (kDisp) {
-    if (!pml)
-      kmdamp_pair(qc, shx, shz, shn, a, b, pa.wpy, out);
-    else
-      cmdamp_pair(qc, shx, shz, shn, a, b, pa.wpy, out);
-    return;
-  }
-  if (!pml) {
-    // KM25ISOQ (estiff25.f:64-154) for the node pair (IAE=a, IBE=b)
-    double me0 = 0.0, me1 = 0.0, me2 = 0.0;
-    double r00 = 0.0, r02 = 0.0, r11 = 0.0, r20 = 0.0, r22 = 0.0;
-    double i01 = 0.0, i10 = 0.0, i12 = 0.0, i21 = 0.0;
-    for (int intx = 0; intx < kNint; intx++)
-      for (int intz = 0; intz < kNint; intz++) {
-        const int q = intx + kNint * intz;
-        const double *c = qc + kNqc * q;
-        const double lambda = c[5], mu = c[6], c11 = c[7], cm1 = c[8], cm2 = c[9];
-        const double wc12 = c[10], wc66 = c[11];
-        const double c13 = lambda, c33 = c11, c55 = mu, c66 = mu, c44 = mu, cm3 = cm1;
-        const double phib = shn[q * kNen + b], phibx = shx[q * kNen + b], phibz = shz[q * kNen + b];
-        const double phia = shn[q * kNen + a], phiax = shx[q * kNen + a], phiaz = shz[q * kNen + a];
-        double phibr1 = phib * cm1, phibr2 = phib * cm2, phibr3 = phib * cm3;
-        double k11t1 = c11 * phibx, k11t2 = c55 * phibz;
-        double k13t1 = c13 * phibz, k13t2 = c55 * phibx;
-        double k22t1 = c66 * phibx, k22t2 = c44 * phibz;
-        double k31t1 = c13 * phibx, k31t2 = c55 * phibz;
-        double k33t1 = c33 * phibz, k33t2 = c55 * phibx;
-        double k12t1 = wc12 * phib, k12t2 = wc66 * phibx;
-        double k21t1 = wc12 * phibx, k21t2 = wc66 * phib;
-        double k23t1 = wc12 * phibz, k23t2 = wc66 * phib;
-        double k32t1 = wc12 * phib, k32t2 = wc66 * phibz;
-        me0 = me0 + phibr1 * phia;
-        me1 = me1 + phibr2 * phia;
-        me2 = me2 + phibr3 * phia;
-        double ke11 = phiax * k11t1 + phiaz * k11t2;
-        double ke13 = phiax * k13t1 + phiaz * k13t2;
-        double ke22 = phiax * k22t1 + phiaz * k22t2;
-        double ke31 = phiaz * k31t1 + phiax * k31t2;
-        double ke33 = phiaz * k33t1 + phiax * k33t2;
-        double ke12 = phiax * k12t1 - phia * k12t2;
-        double ke21 = phia * k21t1 - phiax * k21t2;
-        double ke23 = phia * k23t1 - phiaz * k23t2;
-        double ke32 = phiaz * k32t1 - phia * k32t2;
-        r00 = r00 + ke11;
-        i01 = i01 - ke12;
-        r02 = r02 + ke13;
-        i10 = i10 + ke21;
-        r11 = r11 + ke22;
-        i12 = i12 + ke23;
-        r20 = r20 + ke31;
-        i21 = i21 - ke32;
-        r22 = r22 + ke33;
-      }
-    // ASMBLE_CDIST: R1 = ME + Re(CE), Q1 = Im(CE)
-    out[0] = make_double2(me0 + r00, 0.0);
-    out[1] = make_double2(0.0 + 0.0, i01);
-    out[2] = make_double2(0.0 + r02, 0.0);
-    out[3] = make_double2(0.0 + 0.0, i10);
-    out[4] = make_double2(me1 + r11, 0.0);
-    out[5] = make_double2(0.0 + 0.0, i12);
-    out[6] = make_double2(0.0 + r20, 0.0);
-    out[7] = make_double2(0.0 + 0.0, i21);
-    out[8] = make_double2(me2 + r22, 0.0);
-  } else {
-    // CM25ISOQ (estiff25.f:235-332)
-    const dcx cwpy = dcx{0.0, pa.wpy};
-    double me0 = 0.0, me1 = 0.0, me2 = 0.0;
-    dcx ce[9];
+  if (!pml)
+    kmdamp_pair(qc, shx, shz, shn, a, b, pa.wpy, out);
+  else
+    cmdamp_pair(qc, shx, shz, shn, a, b, pa.wpy, out);
+}
+
+// Non-dispersive element matrices: one CTA of 128 threads per element, a thread
+// takes node b = t % 25 with the five nodes a = 5 (t / 25) + i.  Bound: FP64
+// operations, every multiply and add rounded on its own: 40 a pair and point plus
+// 14 products that depend on b alone, which the five pairs share (54 a pair
+// before).  The shape derivatives live in shared memory (84 KB with the point
+// coefficients; the shape functions themselves, the same for every element, come
+// from the compact global table through L1), so two CTAs share an SM and one
+// computes while the other prepares its points.  A PML element (2.5 times the
+// operations, twice the sums) is two tasks, of three and two nodes a, so that it
+// does not outlast the others of a small launch: task = 2 element + part.
+// 12 000 elements: 4.1 ms against
+// 5.5 ms with one pair a thread and one CTA of 640 an SM.
+constexpr int kTileThreads = 128;
+constexpr int kTileA = 5;    // pairs of a thread
+constexpr int kTileQc = 13;  // coefficient slots per point (odd: no bank conflicts in the set-up)
+constexpr int kTileSm = 2 * kNq * kNen + kTileQc * kNq;
+
+// KM25ISOQ (estiff25.f:64-154) for the node pairs (IAE = a0 + i, IBE = b)
+__device__ __forceinline__ void km25_tile(const double *qc, const double *shx, const double *shz,
+                                          const double *__restrict__ shn, int a0, int b,
+                                          double2 *out) {
+  double me0[kTileA], me1[kTileA], r00[kTileA], r02[kTileA], r11[kTileA], r20[kTileA], r22[kTileA];
+  double i01[kTileA], i10[kTileA], i12[kTileA], i21[kTileA];
 #pragma unroll
-    for (int k = 0; k < 9; k++) ce[k] = dcx{0.0, 0.0};
-    for (int intx = 0; intx < kNint; intx++)
-      for (int intz = 0; intz < kNint; intz++) {
-        const int q = intx + kNint * intz;
-        const double *c = qc + kNqc * q;
-        const double lambda = c[5], mu = c[6], cm1 = c[7], cm2 = c[8], cm3 = cm1;
-        const dcx ex = dcx{c[9], c[10]}, ez = dcx{c[11], c[12]};
-        const dcx clam = dcx{lambda, 0.0}, cmu = dcx{mu, 0.0};
-        const dcx c11 = zadd(zadd(clam, cmu), cmu), c12 = clam, c13 = clam;
-        const dcx c23 = clam, c33 = zadd(zadd(clam, cmu), cmu);
-        const dcx c44 = cmu, c55 = c44, c66 = c44;
-        const double phib = shn[q * kNen + b];
-        const dcx phibx = zmul(dcx{shx[q * kNen + b], 0.0}, ex);
-        const dcx phibz = zmul(dcx{shz[q * kNen + b], 0.0}, ez);
-        double phibr1 = cm1 * phib, phibr2 = cm2 * phib, phibr3 = cm3 * phib;
-        dcx k11t1 = zmul(c11, phibx), k11t2 = zmul(c55, phibz);
-        dcx k13t1 = zmul(c13, phibz), k13t2 = zmul(c55, phibx);
-        dcx k22t1 = zmul(c66, phibx), k22t2 = zmul(c44, phibz);
-        dcx k31t1 = zmul(c13, phibx), k31t2 = zmul(c55, phibz);
-        dcx k33t1 = zmul(c33, phibz), k33t2 = zmul(c55, phibx);
-        dcx k12t1 = zmul(zmul(cwpy, c12), dcx{phib, 0.0});
-        dcx k12t2 = zmul(zmul(cwpy, c66), phibx);
-        dcx k21t1 = zmul(zmul(cwpy, c12), phibx);
-        dcx k21t2 = zmul(zmul(cwpy, c66), dcx{phib, 0.0});
-        dcx k23t1 = zmul(zmul(cwpy, c23), phibz);
-        dcx k23t2 = zmul(zmul(cwpy, c44), dcx{phib, 0.0});
-        dcx k32t1 = zmul(zmul(cwpy, c23), dcx{phib, 0.0});
-        dcx k32t2 = zmul(zmul(cwpy, c44), phibz);
-        const double phia = shn[q * kNen + a];
-        const dcx phiax = zmul(dcx{shx[q * kNen + a], 0.0}, ex);
-        const dcx phiaz = zmul(dcx{shz[q * kNen + a], 0.0}, ez);
-        me0 = me0 + phia * phibr1;
-        me1 = me1 + phia * phibr2;
-        me2 = me2 + phia * phibr3;
-        dcx ce11 = zadd(zmul(phiax, k11t1), zmul(phiaz, k11t2));
-        dcx ce13 = zadd(zmul(phiax, k13t1), zmul(phiaz, k13t2));
-        dcx ce22 = zadd(zmul(phiax, k22t1), zmul(phiaz, k22t2));
-        dcx ce31 = zadd(zmul(phiaz, k31t1), zmul(phiax, k31t2));
-        dcx ce33 = zadd(zmul(phiaz, k33t1), zmul(phiax, k33t2));
-        dcx ce12 = zsub(zmul(phiax, k12t1), zmul(dcx{phia, 0.0}, k12t2));
-        dcx ce21 = zsub(zmul(dcx{phia, 0.0}, k21t1), zmul(phiax, k21t2));
-        dcx ce23 = zsub(zmul(dcx{phia, 0.0}, k23t1), zmul(phiaz, k23t2));
-        dcx ce32 = zsub(zmul(phiaz, k32t1), zmul(dcx{phia, 0.0}, k32t2));
-        ce[0] = zadd(ce[0], ce11);
-        ce[1] = zsub(ce[1], ce12);
-        ce[2] = zadd(ce[2], ce13);
-        ce[3] = zadd(ce[3], ce21);
-        ce[4] = zadd(ce[4], ce22);
-        ce[5] = zadd(ce[5], ce23);
-        ce[6] = zadd(ce[6], ce31);
-        ce[7] = zsub(ce[7], ce32);
-        ce[8] = zadd(ce[8], ce33);
+  for (int i = 0; i < kTileA; i++)
+    me0[i] = me1[i] = r00[i] = r02[i] = r11[i] = r20[i] = r22[i] = i01[i] = i10[i] = i12[i] =
+        i21[i] = 0.0;
+  for (int intx = 0; intx < kNint; intx++)
+    for (int intz = 0; intz < kNint; intz++) {
+      const int q = intx + kNint * intz;
+      const double *c = qc + kTileQc * q;
+      const double lambda = c[5], mu = c[6], c11 = c[7], cm1 = c[8], cm2 = c[9];
+      const double wc12 = c[10], wc66 = c[11];
+      const double phib = __ldg(shn + q * kNen + b), phibx = shx[q * kNen + b],
+                   phibz = shz[q * kNen + b];
+      // the terms of b (C13 = lambda, C33 = C11, C55 = C66 = C44 = mu)
+      const double br1 = phib * cm1, br2 = phib * cm2;
+      const double c11x = c11 * phibx, c11z = c11 * phibz;
+      const double lamx = lambda * phibx, lamz = lambda * phibz;
+      const double mux = mu * phibx, muz = mu * phibz;
+      const double w12n = wc12 * phib, w12x = wc12 * phibx, w12z = wc12 * phibz;
+      const double w66n = wc66 * phib, w66x = wc66 * phibx, w66z = wc66 * phibz;
+#pragma unroll
+      for (int i = 0; i < kTileA; i++) {
+        const int a = q * kNen + a0 + i;
+        const double phia = __ldg(shn + a), phiax = shx[a], phiaz = shz[a];
+        me0[i] = me0[i] + br1 * phia;
+        me1[i] = me1[i] + br2 * phia;
+        const double ke11 = phiax * c11x + phiaz * muz;
+        const double ke13 = phiax * lamz + phiaz * mux;
+        const double ke22 = phiax * mux + phiaz * muz;
+        const double ke31 = phiaz * lamx + phiax * muz;
+        const double ke33 = phiaz * c11z + phiax * mux;
+        const double ke12 = phiax * w12n - phia * w66x;
+        const double ke21 = phia * w12x - phiax * w66n;
+        const double ke23 = phia * w12z - phiaz * w66n;
+        const double ke32 = phiaz * w12n - phia * w66z;
+        r00[i] = r00[i] + ke11;
+        i01[i] = i01[i] - ke12;
+        r02[i] = r02[i] + ke13;
+        i10[i] = i10[i] + ke21;
+        r11[i] = r11[i] + ke22;
+        i12[i] = i12[i] + ke23;
+        r20[i] = r20[i] + ke31;
+        i21[i] = i21[i] - ke32;
+        r22[i] = r22[i] + ke33;
       }
-    out[0] = make_double2(me0 + ce[0].re, ce[0].im);
-    out[1] = make_double2(0.0 + ce[1].re, ce[1].im);
-    out[2] = make_double2(0.0 + ce[2].re, ce[2].im);
-    out[3] = make_double2(0.0 + ce[3].re, ce[3].im);
-    out[4] = make_double2(me1 + ce[4].re, ce[4].im);
-    out[5] = make_double2(0.0 + ce[5].re, ce[5].im);
-    out[6] = make_double2(0.0 + ce[6].re, ce[6].im);
-    out[7] = make_double2(0.0 + ce[7].re, ce[7].im);
-    out[8] = make_double2(me2 + ce[8].re, ce[8].im);
+    }
+  // ASMBLE_CDIST: R1 = ME + Re(CE), Q1 = Im(CE); ME is the same on (1,1) and (3,3)
+#pragma unroll
+  for (int i = 0; i < kTileA; i++) {
+    double2 *o = out + (size_t)((a0 + i) * kNen + b) * 9;
+    o[0] = make_double2(me0[i] + r00[i], 0.0);
+    o[1] = make_double2(0.0 + 0.0, i01[i]);
+    o[2] = make_double2(0.0 + r02[i], 0.0);
+    o[3] = make_double2(0.0 + 0.0, i10[i]);
+    o[4] = make_double2(me1[i] + r11[i], 0.0);
+    o[5] = make_double2(0.0 + 0.0, i12[i]);
+    o[6] = make_double2(0.0 + r20[i], 0.0);
+    o[7] = make_double2(0.0 + 0.0, i21[i]);
+    o[8] = make_double2(me0[i] + r22[i], 0.0);
+  }
+}
+
+// CM25ISOQ (estiff25.f:235-332) for NA node pairs.  The reference multiplies
+// complex numbers throughout; where an operand is purely real or imaginary (the
+// moduli, the shape functions, i omega py) only the products that are not exact
+// zeros are formed.  Adding a zero product changes no finite sum (the sums start
+// at +0, so no zero's sign survives either).
+template <int NA>
+__device__ __forceinline__ void cm25_tile(const double *qc, const double *shx, const double *shz,
+                                          const double *__restrict__ shn, int a0, int b,
+                                          double wpy, double2 *out) {
+  double me0[NA], me1[NA];
+  dcx ce[9][NA];
+#pragma unroll
+  for (int i = 0; i < NA; i++) {
+    me0[i] = me1[i] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) ce[k][i] = dcx{0.0, 0.0};
+  }
+  for (int intx = 0; intx < kNint; intx++)
+    for (int intz = 0; intz < kNint; intz++) {
+      const int q = intx + kNint * intz;
+      const double *c = qc + kTileQc * q;
+      const double lam = c[5], mu = c[6], cm1 = c[7], cm2 = c[8];
+      const dcx ex = dcx{c[9], c[10]}, ez = dcx{c[11], c[12]};
+      const double c11 = lam + mu + mu, wl = wpy * lam, wm = wpy * mu;
+      const double phib = __ldg(shn + q * kNen + b), sxb = shx[q * kNen + b], szb = shz[q * kNen + b];
+      const dcx bx = dcx{sxb * ex.re, sxb * ex.im}, bz = dcx{szb * ez.re, szb * ez.im};
+      const double br1 = cm1 * phib, br2 = cm2 * phib;
+      const dcx c11x = dcx{c11 * bx.re, c11 * bx.im}, c11z = dcx{c11 * bz.re, c11 * bz.im};
+      const dcx lamx = dcx{lam * bx.re, lam * bx.im}, lamz = dcx{lam * bz.re, lam * bz.im};
+      const dcx mux = dcx{mu * bx.re, mu * bx.im}, muz = dcx{mu * bz.re, mu * bz.im};
+      const double wln = wl * phib, wmn = wm * phib;  // times i
+      const dcx wlx = dcx{-(wl * bx.im), wl * bx.re}, wlz = dcx{-(wl * bz.im), wl * bz.re};
+      const dcx wmx = dcx{-(wm * bx.im), wm * bx.re}, wmz = dcx{-(wm * bz.im), wm * bz.re};
+#pragma unroll
+      for (int i = 0; i < NA; i++) {
+        const int a = q * kNen + a0 + i;
+        const double phia = __ldg(shn + a), sxa = shx[a], sza = shz[a];
+        const dcx ax = dcx{sxa * ex.re, sxa * ex.im}, az = dcx{sza * ez.re, sza * ez.im};
+        me0[i] = me0[i] + phia * br1;
+        me1[i] = me1[i] + phia * br2;
+        ce[0][i] = zadd(ce[0][i], zadd(zmul(ax, c11x), zmul(az, muz)));
+        ce[2][i] = zadd(ce[2][i], zadd(zmul(ax, lamz), zmul(az, mux)));
+        ce[4][i] = zadd(ce[4][i], zadd(zmul(ax, mux), zmul(az, muz)));
+        ce[6][i] = zadd(ce[6][i], zadd(zmul(az, lamx), zmul(ax, muz)));
+        ce[8][i] = zadd(ce[8][i], zadd(zmul(az, c11z), zmul(ax, mux)));
+        ce[1][i] = zsub(ce[1][i], zsub(dcx{-(ax.im * wln), ax.re * wln},
+                                       dcx{phia * wmx.re, phia * wmx.im}));
+        ce[3][i] = zadd(ce[3][i], zsub(dcx{phia * wlx.re, phia * wlx.im},
+                                       dcx{-(ax.im * wmn), ax.re * wmn}));
+        ce[5][i] = zadd(ce[5][i], zsub(dcx{phia * wlz.re, phia * wlz.im},
+                                       dcx{-(az.im * wmn), az.re * wmn}));
+        ce[7][i] = zsub(ce[7][i], zsub(dcx{-(az.im * wln), az.re * wln},
+                                       dcx{phia * wmz.re, phia * wmz.im}));
+      }
+    }
+#pragma unroll
+  for (int i = 0; i < NA; i++) {
+    double2 *o = out + (size_t)((a0 + i) * kNen + b) * 9;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const double m = k == 0 || k == 8 ? me0[i] : k == 4 ? me1[i] : 0.0;
+      o[k] = make_double2(m + ce[k][i].re, ce[k][i].im);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kTileThreads, 2)
+    k_elem_plain(MeshView mv, DevTables dt, PlainArgs pa, const int *__restrict__ tasks,
+                 double2 *__restrict__ elemmat, int *__restrict__ err) {
+  extern __shared__ double sm[];
+  double *shx = sm, *shz = sm + kNq * kNen, *qc = sm + 2 * kNq * kNen;
+  const int task = tasks[blockIdx.x], e = task >> 1;
+  const int t = threadIdx.x;
+  const int4 ie = mv.ieng[e];
+  const bool pml = mv.cdomain[e] == 'A';
+  // ---- per quadrature point: Jacobian, interpolated model, coefficients
+  for (int q = t; q < kNq; q += kTileThreads) {
+    const int intx = q % kNint, intz = q / kNint;
+    QGeo g;
+    if (!quad_geo(mv, dt, ie, q, pml, g)) atomicCAS(err, 0, e + 1);
+    double *c = qc + kTileQc * q;
+    c[0] = g.dxdxi; c[1] = g.dxdeta; c[2] = g.dzdxi; c[3] = g.dzdeta; c[4] = g.rjac;
+    const double weight = dt.wts[intx] * dt.wts[intz] * g.rjac;
+    const double lambda = g.lam * weight, mu = g.mu * weight, rhow = g.rho * weight;
+    c[5] = lambda;
+    c[6] = mu;
+    if (!pml) {
+      const double c11 = lambda + 2.0 * mu;
+      c[7] = c11;
+      c[8] = -pa.w2 * (rhow - pa.py2 * mu);   // COEFFM1 (C66)
+      c[9] = -pa.w2 * (rhow - pa.py2 * c11);  // COEFFM2 (C22)
+      c[10] = pa.wpy * lambda;                // WPY*C12 = WPY*C23
+      c[11] = pa.wpy * mu;                    // WPY*C66 = WPY*C44
+    } else {
+      dcx ex = dcx{1.0, 0.0}, ez = dcx{1.0, 0.0};
+      if (g.xdep > 2.22e-16)
+        ex = zdampfn(g.xdep, g.vel, pa.pml.xwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
+                     pa.pml.fcent, pa.omega);
+      if (g.zdep > 2.22e-16)
+        ez = zdampfn(g.zdep, g.vel, pa.pml.zwidth, pa.pml.dmax, pa.logr, pa.pml.kappa,
+                     pa.pml.fcent, pa.omega);
+      c[7] = -pa.w2 * (rhow - pa.py2 * mu);                  // COEFFM1
+      c[8] = -pa.w2 * (rhow - pa.py2 * (lambda + 2.0 * mu)); // COEFFM2
+      c[9] = ex.re; c[10] = ex.im;
+      c[11] = ez.re; c[12] = ez.im;
+    }
+  }
+  __syncthreads();
+  // ---- global shape-function derivatives (CJMK_TVI cjac.f:128-134)
+#pragma unroll 4
+  for (int idx = t; idx < kNq * kNen; idx += kTileThreads) {
+    const double *c = qc + kTileQc * (idx / kNen);
+    const double *sl = dt.shl + 3 * (size_t)idx;
+    const double drnxi = sl[0], drneta = sl[1];
+    shx[idx] = (drnxi * c[3] - drneta * c[2]) / c[4];
+    shz[idx] = -(drnxi * c[1] - drneta * c[0]) / c[4];
+  }
+  __syncthreads();
+  if (t >= kNen * kNl) return;
+  const int a0 = kTileA * (t / kNen), b = t % kNen;
+  double2 *out = elemmat + (size_t)e * kNab * 9;
+  if (!pml) {
+    km25_tile(qc, shx, shz, dt.shn, a0, b, out);
+  } else if ((task & 1) == 0) {
+    cm25_tile<3>(qc, shx, shz, dt.shn, a0, b, pa.wpy, out);
+  } else {
+    cm25_tile<2>(qc, shx, shz, dt.shn, a0 + 3, b, pa.wpy, out);
   }
 }
 
@@ -485,22 +543,43 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
 // Sum of the element contributions of every nonzero of [nz0, nz1) in element order:
 // FP64 (complex128 output) and the reference's COMPLEX*8 accumulation
 // CDIST = CDIST + CMPLX(CARG) (asmble.f90:302-305).
-__global__ void k_gather_plain(long long nz0, long long nz1, const int *__restrict__ gptr,
-                               const int *__restrict__ glist, const double2 *__restrict__ elemmat,
-                               double2 *__restrict__ csr128, float2 *__restrict__ csr64) {
-  long long nz = nz0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (nz >= nz1) return;
-  double sr = 0.0, si = 0.0;
-  float fr = 0.0f, fi = 0.0f;
-  for (int k = gptr[nz]; k < gptr[nz + 1]; k++) {
-    double2 v = elemmat[glist[k]];
-    sr = sr + v.x;
-    si = si + v.y;
-    fr = fr + __double2float_rn(v.x);
-    fi = fi + __double2float_rn(v.y);
+// Bound: HBM (24 bytes written, about 26 read a nonzero).  Four nonzeros a thread,
+// a CTA's width apart: their list bounds, first contributions' places and values
+// are each in flight together; 61.6 M nonzeros: 595 us against 800 one by one.
+constexpr int kGatherThreads = 256, kGatherPer = 4;
+__global__ void __launch_bounds__(kGatherThreads)
+    k_gather_plain(long long nz0, long long nz1, const int *__restrict__ gptr,
+                   const int *__restrict__ glist, const double2 *__restrict__ elemmat,
+                   double2 *__restrict__ csr128, float2 *__restrict__ csr64) {
+  const long long base = nz0 + (long long)blockIdx.x * kGatherThreads * kGatherPer + threadIdx.x;
+  int b[kGatherPer], n[kGatherPer], at[kGatherPer];
+  double2 v0[kGatherPer];
+#pragma unroll
+  for (int u = 0; u < kGatherPer; u++) {
+    const long long nz = base + u * kGatherThreads;
+    b[u] = nz < nz1 ? gptr[nz] : 0;
+    n[u] = nz < nz1 ? gptr[nz + 1] - b[u] : 0;
   }
-  if (csr128) csr128[nz] = make_double2(sr, si);
-  if (csr64) csr64[nz] = make_float2(fr, fi);
+#pragma unroll
+  for (int u = 0; u < kGatherPer; u++) at[u] = n[u] > 0 ? glist[b[u]] : 0;
+#pragma unroll
+  for (int u = 0; u < kGatherPer; u++) v0[u] = n[u] > 0 ? elemmat[at[u]] : make_double2(0.0, 0.0);
+#pragma unroll
+  for (int u = 0; u < kGatherPer; u++) {
+    const long long nz = base + u * kGatherThreads;
+    if (nz >= nz1) continue;
+    double sr = 0.0, si = 0.0;
+    float fr = 0.0f, fi = 0.0f;
+    for (int k = 0; k < n[u]; k++) {
+      const double2 v = k == 0 ? v0[u] : elemmat[glist[b[u] + k]];
+      sr = sr + v.x;
+      si = si + v.y;
+      fr = fr + __double2float_rn(v.x);
+      fi = fi + __double2float_rn(v.y);
+    }
+    if (csr128) csr128[nz] = make_double2(sr, si);
+    if (csr64) csr64[nz] = make_float2(fr, fi);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -612,19 +691,23 @@ cudaError_t launch_elem_plain(Ctx *c, char cftype, double freq, double py, int e
   pa.freq0 = c->mesh_scalars.freq0;
   pa.fac1 = (pa.ldisp && pa.freq0 != 0.0) ? std::log(freq / pa.freq0) : 0.0;
   pa.ebase = e0;
-  size_t smem = sizeof(double) * kSmTot;
   if (pa.ldisp) {
-    cudaError_t e = cudaFuncSetAttribute(k_elem_plain<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = sizeof(double) * kSmTot;
+    cudaError_t e = cudaFuncSetAttribute(k_elem_disp, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
     if (e != cudaSuccess) return e;
-    k_elem_plain<true><<<e1 - e0, kPlainThreads, smem, st>>>(c->mv, c->dt, pa, c->d_elemmat,
-                                                             c->d_err);
+    k_elem_disp<<<e1 - e0, kPlainThreads, smem, st>>>(c->mv, c->dt, pa, c->d_elemmat, c->d_err);
   } else {
-    cudaError_t e = cudaFuncSetAttribute(k_elem_plain<false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = sizeof(double) * kTileSm;
+    cudaError_t e = cudaFuncSetAttribute(k_elem_plain, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
     if (e != cudaSuccess) return e;
-    k_elem_plain<false><<<e1 - e0, kPlainThreads, smem, st>>>(c->mv, c->dt, pa, c->d_elemmat,
-                                                              c->d_err);
+    const int t0 = c->h_task0[e0], t1 = c->h_task0[e1];
+    // a launch over the whole mesh takes the PML elements first, so that none of
+    // them ends it alone
+    const int *tasks = t1 - t0 == c->h_task0[c->nelem] ? c->d_tasks_pml : c->d_tasks + t0;
+    k_elem_plain<<<t1 - t0, kTileThreads, smem, st>>>(c->mv, c->dt, pa, tasks, c->d_elemmat,
+                                                      c->d_err);
   }
   return cudaGetLastError();
 }
@@ -633,10 +716,9 @@ cudaError_t launch_elem_plain(Ctx *c, char cftype, double freq, double py, int e
 cudaError_t launch_gather_plain(Ctx *c, double *csr128, float *csr64, long long nz0,
                                 long long nz1, cudaStream_t st) {
   if (nz1 <= nz0) return cudaSuccess;
-  int th = 256;
-  long long blocks = (nz1 - nz0 + th - 1) / th;
-  k_gather_plain<<<(unsigned)blocks, th, 0, st>>>(nz0, nz1, c->d_gptr, c->d_glist, c->d_elemmat,
-                                                   (double2 *)csr128, (float2 *)csr64);
+  const long long per = kGatherThreads * kGatherPer, blocks = (nz1 - nz0 + per - 1) / per;
+  k_gather_plain<<<(unsigned)blocks, kGatherThreads, 0, st>>>(
+      nz0, nz1, c->d_gptr, c->d_glist, c->d_elemmat, (double2 *)csr128, (float2 *)csr64);
   return cudaGetLastError();
 }
 
