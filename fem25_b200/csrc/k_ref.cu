@@ -489,32 +489,44 @@ cudaError_t launch_misfit_part(Ctx *c, int nsrc, int nrec, const int *d_mrdof, c
 // ---------------------------------------------------------------------------
 // reference-compatible virtual forces: one CTA per CSC column (inversion
 // anchor), elements of MCONN in order.  DKM_VPVS (dstiff25.f:498-662) is
-// evaluated by 625 threads (node pairs) into shared memory as COMPLEX*8
-// CARG = CMPLX(DCMPLX(DME) + DKE) (vforce25.f:311-312), then 75 threads form
-// FORCEV(row) += CARG * WAVE * CWGHT in IQE order (vforce25.f:326-330).
+// evaluated into shared memory as COMPLEX*8 CARG = CMPLX(DCMPLX(DME) + DKE)
+// (vforce25.f:311-312), whose imaginary part is zero in every entry, then 75
+// threads form FORCEV(row) += CARG * WAVE * CWGHT in IQE order
+// (vforce25.f:326-330).
+// Bound: FP64 operations, rounded one by one.  A thread takes node b = t % 25
+// with the five nodes a = 5 (t / 25) + i: the 17 products that depend on b alone
+// serve five pairs (52 operations a pair and point beside them, 68 before), and
+// 81 KB of shared memory (CARG takes the place of the shape derivatives) let two
+// CTAs share an SM, one summing while the other prepares.  11 000 anchors:
+// 5.1 ms against 7.2 ms with one pair a thread and one CTA of 640 an SM.
 // ---------------------------------------------------------------------------
 constexpr int kRefThreads = 640;
+constexpr int kCfThreads = 128, kCfA = 5;
+constexpr int kCfQc = 13;  // geometry 0-4, then the operator's point coefficients
+constexpr int kCfSm = 2 * kNq * kNen + kCfQc * kNq;
 
 struct RefArgs {
   double omega, py, vpvs2;
   int lisp, accumulate, ncon, nnpg;
 };
 
-__global__ void __launch_bounds__(kRefThreads, 1)
+__global__ void __launch_bounds__(kCfThreads, 2)
     k_ref_cfmat(MeshView mv, DevTables dt, RefArgs ra, const int *__restrict__ lm,
                 const int *__restrict__ anchor_of_col, const int *__restrict__ mconn,
                 const double *__restrict__ elem_wts, const int *__restrict__ jcsc,
                 const int *__restrict__ icsc, const float2 *__restrict__ wave,
                 float2 *__restrict__ fmat, int *__restrict__ err) {
   extern __shared__ double sm[];
-  double *shx = sm, *shz = sm + kNq * kNen, *shn = sm + 2 * kNq * kNen;
-  double *qc = sm + 3 * kNq * kNen;                       // [kNq][8]
-  float2 *carg = reinterpret_cast<float2 *>(qc + 8 * kNq); // [75][75]
+  double *shx = sm, *shz = sm + kNq * kNen;
+  double *qc = sm + 2 * kNq * kNen;             // [kNq][kCfQc]
+  float *carg = reinterpret_cast<float *>(sm);  // [75][75], real parts, over shx / shz
+  __shared__ float2 wv[kNee];
+  __shared__ int dof[kNee];
   const int col = blockIdx.x, t = threadIdx.x;
   const int p = anchor_of_col[col];  // 0-based anchor (INPG-1)
   const int i1 = jcsc[col] - 1, i2 = jcsc[col + 1] - 1, nnzrow = i2 - i1;
   float2 *forcev = fmat + i1;
-  for (int k = t; k < nnzrow; k += kRefThreads) forcev[k] = make_float2(0.0f, 0.0f);
+  for (int k = t; k < nnzrow; k += kCfThreads) forcev[k] = make_float2(0.0f, 0.0f);
   // elements of the anchor, in MCONN order; without accumulation only the
   // last one leaves a trace in FORCEV
   int elist[8], ne = 0;
@@ -529,8 +541,13 @@ __global__ void __launch_bounds__(kRefThreads, 1)
   for (int ie_ = first; ie_ < ne; ie_++) {
     const int e = elist[ie_];
     const int4 ie = mv.ieng[e];
-    if (t < kNq) {
-      const int q = t, intx = q % kNint, intz = q / kNint;
+    for (int k = t; k < kNee; k += kCfThreads) {
+      const int d = lm[(size_t)e * kNee + k];
+      dof[k] = d;
+      wv[k] = d > 0 ? wave[d - 1] : make_float2(0.0f, 0.0f);
+    }
+    for (int q = t; q < kNq; q += kCfThreads) {
+      const int intx = q % kNint, intz = q / kNint;
       QGeo g;
       if (!quad_geo(mv, dt, ie, q, false, g)) atomicCAS(err, 0, e + 1);
       // DJACAB (djac.f:90-110): DAB = sum_ia 2 alpha_ia SF(ia), alpha nonzero
@@ -554,82 +571,93 @@ __global__ void __launch_bounds__(kRefThreads, 1)
         dvp = dab2 * ra.vpvs2;
         dvs = dab2;
       }
-      double *c = qc + 8 * q;
+      double *c = qc + kCfQc * q;
       c[0] = g.dxdxi; c[1] = g.dxdeta; c[2] = g.dzdxi; c[3] = g.dzdeta; c[4] = g.rjac;
-      double weight = dt.wts[intx] * dt.wts[intz] * g.rjac;
-      c[5] = dvp * weight;  // DRVP
-      c[6] = dvs * weight;  // DRVS
+      const double weight = dt.wts[intx] * dt.wts[intz] * g.rjac;
+      const double drvp = dvp * weight, drvs = dvs * weight;
+      c[5] = drvp;
+      c[6] = drvs;
+      c[7] = w2 * py2 * drvs;    // RMCOEFF1
+      c[8] = w2 * py2 * drvp;    // RMCOEFF2
+      c[9] = -2.0 * drvs;
+      c[10] = wpy * drvp;
+      c[11] = -2.0 * wpy * drvs;
+      c[12] = -wpy * drvs;
     }
     __syncthreads();
-    for (int idx = t; idx < kNq * kNen; idx += kRefThreads) {
-      const int q = idx / kNen;
-      const double *c = qc + 8 * q;
+#pragma unroll 4
+    for (int idx = t; idx < kNq * kNen; idx += kCfThreads) {
+      const double *c = qc + kCfQc * (idx / kNen);
       const double *sl = dt.shl + 3 * (size_t)idx;
-      double drnxi = sl[0], drneta = sl[1];
+      const double drnxi = sl[0], drneta = sl[1];
       shx[idx] = (drnxi * c[3] - drneta * c[2]) / c[4];
       shz[idx] = -(drnxi * c[1] - drneta * c[0]) / c[4];
-      shn[idx] = sl[2];
     }
     __syncthreads();
-    if (t < kNab) {
-      const int a = t / kNen, b = t % kNen;
-      double m0 = 0.0, m1 = 0.0, m2 = 0.0;
-      double r00 = 0.0, r11 = 0.0, r22 = 0.0, r02 = 0.0, r20 = 0.0;
-      double r01 = 0.0, r10 = 0.0, r12 = 0.0, r21 = 0.0;
+    const bool on = t < kNen * kNl;
+    const int a0 = kCfA * (t / kNen), b = t % kNen;
+    double m0[kCfA], m1[kCfA], r00[kCfA], r11[kCfA], r22[kCfA], r02[kCfA], r20[kCfA];
+    double r01[kCfA], r10[kCfA], r12[kCfA], r21[kCfA];
+#pragma unroll
+    for (int i = 0; i < kCfA; i++)
+      m0[i] = m1[i] = r00[i] = r11[i] = r22[i] = r02[i] = r20[i] = r01[i] = r10[i] = r12[i] =
+          r21[i] = 0.0;
+    if (on) {
       for (int intx = 0; intx < kNint; intx++)
         for (int intz = 0; intz < kNint; intz++) {
           const int q = intx + kNint * intz;
-          const double drvp = qc[8 * q + 5], drvs = qc[8 * q + 6];
-          const double rm1 = w2 * py2 * drvs, rm2 = w2 * py2 * drvp;
-          const double phib = shn[q * kNen + b], phibx = shx[q * kNen + b], phibz = shz[q * kNen + b];
-          const double phia = shn[q * kNen + a], phiax = shx[q * kNen + a], phiaz = shz[q * kNen + a];
-          double rm11t1 = rm1 * phib, rm22t1 = rm2 * phib;
-          double rk11t1 = drvp * phibx, rk11t2 = drvs * phibz;
-          double rk13t1 = drvp * phibz, rk13t2 = drvs * phibx, rk13t3 = -2.0 * drvs * phibz;
-          double rk22t1 = drvs * phibx, rk22t2 = drvs * phibz;
-          double rk31t1 = drvp * phibx, rk31t2 = drvs * phibz, rk31t3 = -2.0 * drvs * phibx;
-          double rk33t1 = drvp * phibz, rk33t2 = drvs * phibx;
-          double rk12t1 = wpy * drvp * phib, rk12t2 = -2.0 * wpy * drvs * phib, rk12t3 = -wpy * drvs * phibx;
-          double rk21t1 = wpy * drvp * phibx, rk21t2 = -2.0 * wpy * drvs * phibx, rk21t3 = -wpy * drvs * phib;
-          double rk23t1 = wpy * drvp * phibz, rk23t2 = -2.0 * wpy * drvs * phibz, rk23t3 = -wpy * drvs * phib;
-          double rk32t1 = wpy * drvp * phib, rk32t2 = -2.0 * wpy * drvs * phib, rk32t3 = -wpy * drvs * phibz;
-          double rme11 = rm11t1 * phia, rme22 = rm22t1 * phia, rme33 = rme11;
-          m0 = m0 + rme11;
-          m1 = m1 + rme22;
-          m2 = m2 + rme33;
-          r00 = r00 + (rk11t1 * phiax + rk11t2 * phiaz);
-          r11 = r11 + (rk22t1 * phiax + rk22t2 * phiaz);
-          r22 = r22 + (rk33t1 * phiaz + rk33t2 * phiax);
-          r02 = r02 + (rk13t1 * phiax + rk13t2 * phiaz + rk13t3 * phiax);
-          r20 = r20 + (rk31t1 * phiaz + rk31t2 * phiax + rk31t3 * phiaz);
-          r01 = r01 - (rk12t1 * phiax + rk12t2 * phiax + rk12t3 * phia);
-          r10 = r10 + (rk21t1 * phia + rk21t2 * phia + rk21t3 * phiax);
-          r12 = r12 + (rk23t1 * phia + rk23t2 * phia + rk23t3 * phiaz);
-          r21 = r21 - (rk32t1 * phiaz + rk32t2 * phiaz + rk32t3 * phia);
+          const double *c = qc + kCfQc * q;
+          const double drvp = c[5], drvs = c[6], rm1 = c[7], rm2 = c[8];
+          const double m2s = c[9], wp = c[10], m2ws = c[11], mws = c[12];
+          const double phib = __ldg(dt.shn + q * kNen + b);
+          const double phibx = shx[q * kNen + b], phibz = shz[q * kNen + b];
+          const double rm1n = rm1 * phib, rm2n = rm2 * phib;
+          const double px = drvp * phibx, pz = drvp * phibz;
+          const double sx = drvs * phibx, sz = drvs * phibz;
+          const double m2x = m2s * phibx, m2z = m2s * phibz;
+          const double wpn = wp * phib, wpx = wp * phibx, wpz = wp * phibz;
+          const double m2n = m2ws * phib, m2wx = m2ws * phibx, m2wz = m2ws * phibz;
+          const double mwn = mws * phib, mwx = mws * phibx, mwz = mws * phibz;
+#pragma unroll
+          for (int i = 0; i < kCfA; i++) {
+            const int a = q * kNen + a0 + i;
+            const double phia = __ldg(dt.shn + a), phiax = shx[a], phiaz = shz[a];
+            m0[i] = m0[i] + rm1n * phia;  // DME(1,1) = DME(3,3)
+            m1[i] = m1[i] + rm2n * phia;
+            r00[i] = r00[i] + (px * phiax + sz * phiaz);
+            r11[i] = r11[i] + (sx * phiax + sz * phiaz);
+            r22[i] = r22[i] + (pz * phiaz + sx * phiax);
+            r02[i] = r02[i] + (pz * phiax + sx * phiaz + m2z * phiax);
+            r20[i] = r20[i] + (px * phiaz + sz * phiax + m2x * phiaz);
+            r01[i] = r01[i] - (wpn * phiax + m2n * phiax + mwx * phia);
+            r10[i] = r10[i] + (wpx * phia + m2wx * phia + mwn * phiax);
+            r12[i] = r12[i] + (wpz * phia + m2wz * phia + mwn * phiaz);
+            r21[i] = r21[i] - (wpn * phiaz + m2n * phiaz + mwz * phia);
+          }
         }
-      // CARG = CMPLX(DCMPLX(DME,0) + DKE): DKE is real in every entry
-      const int ipe = 3 * a, iqe = 3 * b;
-      float2 *row0 = carg + (size_t)ipe * kNee + iqe;
-      row0[0] = make_float2(__double2float_rn(m0 + r00), __double2float_rn(0.0 + 0.0));
-      row0[1] = make_float2(__double2float_rn(0.0 + r01), __double2float_rn(0.0 + 0.0));
-      row0[2] = make_float2(__double2float_rn(0.0 + r02), __double2float_rn(0.0 + 0.0));
-      float2 *row1 = row0 + kNee;
-      row1[0] = make_float2(__double2float_rn(0.0 + r10), __double2float_rn(0.0 + 0.0));
-      row1[1] = make_float2(__double2float_rn(m1 + r11), __double2float_rn(0.0 + 0.0));
-      row1[2] = make_float2(__double2float_rn(0.0 + r12), __double2float_rn(0.0 + 0.0));
-      float2 *row2 = row1 + kNee;
-      row2[0] = make_float2(__double2float_rn(0.0 + r20), __double2float_rn(0.0 + 0.0));
-      row2[1] = make_float2(__double2float_rn(0.0 + r21), __double2float_rn(0.0 + 0.0));
-      row2[2] = make_float2(__double2float_rn(m2 + r22), __double2float_rn(0.0 + 0.0));
     }
-    __syncthreads();
+    __syncthreads();  // every read of the shape derivatives is done
+    if (on) {
+#pragma unroll
+      for (int i = 0; i < kCfA; i++) {
+        float *row0 = carg + (3 * (a0 + i)) * kNee + 3 * b, *row1 = row0 + kNee, *row2 = row1 + kNee;
+        row0[0] = __double2float_rn(m0[i] + r00[i]);
+        row0[1] = __double2float_rn(0.0 + r01[i]);
+        row0[2] = __double2float_rn(0.0 + r02[i]);
+        row1[0] = __double2float_rn(0.0 + r10[i]);
+        row1[1] = __double2float_rn(m1[i] + r11[i]);
+        row1[2] = __double2float_rn(0.0 + r12[i]);
+        row2[0] = __double2float_rn(0.0 + r20[i]);
+        row2[1] = __double2float_rn(0.0 + r21[i]);
+        row2[2] = __double2float_rn(m0[i] + r22[i]);
+      }
+    }
     if (!ra.accumulate)
-      for (int k = t; k < nnzrow; k += kRefThreads) forcev[k] = make_float2(0.0f, 0.0f);
+      for (int k = t; k < nnzrow; k += kCfThreads) forcev[k] = make_float2(0.0f, 0.0f);
     __syncthreads();
     if (t < kNee) {
       const int ipe = t;
-      const int *lme = lm + (size_t)e * kNee;
-      const int idof = lme[ipe];
+      const int idof = dof[ipe];
       if (idof > 0) {
         // IBSECT on the CSC column
         int lo = 0, hi = nnzrow - 1, inz = -1;
@@ -645,11 +673,10 @@ __global__ void __launch_bounds__(kRefThreads, 1)
           const float cw = __double2float_rn(elem_wts[e]);
           float fr = forcev[inz].x, fi = forcev[inz].y;
           for (int iqe = 0; iqe < kNee; iqe++) {
-            const int jdof = lme[iqe];
-            if (jdof <= 0) continue;
-            const float2 cv = carg[(size_t)ipe * kNee + iqe], wv = wave[jdof - 1];
-            cfl t1 = cmulf(cfl{cv.x, cv.y}, cfl{wv.x, wv.y});
-            cfl t2 = cmulf(t1, cfl{cw, 0.0f});
+            if (dof[iqe] <= 0) continue;
+            const float2 w = wv[iqe];
+            const cfl t1 = cmulf(cfl{carg[ipe * kNee + iqe], 0.0f}, cfl{w.x, w.y});
+            const cfl t2 = cmulf(t1, cfl{cw, 0.0f});
             fr = fr + t2.re;
             fi = fi + t2.im;
           }
@@ -1179,10 +1206,6 @@ __global__ void k_ref_adjflam(int ncol, const int *__restrict__ jcsc, const int 
   gradl[k] = gradl[k] + (-1.0f) * v;
 }
 
-static size_t ref_smem() {
-  return sizeof(double) * (3 * kNq * kNen + 8 * kNq) + sizeof(float2) * kNee * kNee;
-}
-
 cudaError_t launch_ref_cfmat(Ctx *c, int lisp, double vpvs, double omega, double py,
                              const float *wave, int accumulate, cudaStream_t st) {
   RefArgs ra;
@@ -1194,9 +1217,9 @@ cudaError_t launch_ref_cfmat(Ctx *c, int lisp, double vpvs, double omega, double
   ra.ncon = c->rg.ncon;
   ra.nnpg = c->nnpg;
   cudaError_t e = cudaFuncSetAttribute(k_ref_cfmat, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)ref_smem());
+                                       (int)(sizeof(double) * kCfSm));
   if (e) return e;
-  k_ref_cfmat<<<c->rg.nnpinv, kRefThreads, ref_smem(), st>>>(
+  k_ref_cfmat<<<c->rg.nnpinv, kCfThreads, sizeof(double) * kCfSm, st>>>(
       c->mv, c->dt, ra, c->d_lm, c->d_rg_anchor, c->d_mconn, c->d_elem_wts, c->d_jcsc, c->d_icsc,
       (const float2 *)wave, c->d_fmat, c->d_err);
   return cudaGetLastError();
