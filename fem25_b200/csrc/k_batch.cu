@@ -90,72 +90,165 @@ __global__ void __launch_bounds__(kElemThreads, 1)
 // Per PML element node pair at one omega: the 9 complex CE coefficients
 // (CE0 on the (1,1),(1,3),(2,2),(3,1),(3,3) blocks, CE1 -- the coefficient of
 // omega*py -- on the others), entry k = 3i+j.
-__global__ void __launch_bounds__(kElemThreads, 1)
-    k_elem_pml(MeshView mv, DevTables dt, const int *__restrict__ pml_elems, PmlParams pp,
-               double logr, double2 *__restrict__ pemat, int *__restrict__ err) {
+// Bound: FP64 operations.  With the shape functions' factors l_ix(xi) l_iz(eta),
+// every block is a sum over four kinds of term (a, b differentiated along xi or
+// eta, or not at all)
+//   sum_qz s_iz(qz) t_jz(qz) sum_qx c(qx, qz) p_ix(qx) r_jx(qx),   p, r, s, t = l or l'
+// with the stretched metric, the moduli and the weights in c, so the two sums are
+// taken one after the other: 0.9 M multiply-adds an element instead of 7 M over
+// node pairs and points.  A CTA takes one block row of an element (its stages are
+// short and wait for one another, so more CTAs hide more), block by block: c of the
+// four kinds by points, the xi sums by (kind, qz, ix) for five jx, the eta sums by
+// (two kinds, ix, jx, iz) for five jz.  318 elements: 84 us against 300.
+constexpr int kPmlThreads = 288;
+struct PmlPoint {
+  double x[2], z[2];  // d xi / d x, d eta / d x; d xi / d z, d eta / d z
+  double lam, mu;     // times the weight and the Jacobian
+  dcx ex, ez;
+};
+__device__ __forceinline__ dcx zscale(double f, dcx a) { return dcx{f * a.re, f * a.im}; }
+__global__ void __launch_bounds__(kPmlThreads, 3)
+    k_elem_pml(MeshView mv, DevTables dt, ShapeTabs tb, const int *__restrict__ pml_elems,
+               PmlParams pp, double logr, double2 *__restrict__ pemat, int *__restrict__ err) {
+  constexpr int kLine = kNl * kNl * kNint;  // xi sums of one kind: [ix][jx][qz]
   extern __shared__ double sm[];
-  double *shx = sm, *shz = sm + kNq * kNen, *qc = sm + 2 * kNq * kNen;
+  double2 *c = reinterpret_cast<double2 *>(sm);            // [4][kNq]
+  double2 *g = c + 4 * kNq;                                // [4][kLine]
+  double2 *half = g + 4 * kLine;                           // [kNab]
+  PmlPoint *pt = reinterpret_cast<PmlPoint *>(half + kNab);  // [kNq]
+  double *tab[2] = {reinterpret_cast<double *>(pt + kNq),
+                    reinterpret_cast<double *>(pt + kNq) + kNint * kNl};  // l, l'
   const int pe = blockIdx.x, e = pml_elems[pe], t = threadIdx.x;
   const int4 ie = mv.ieng[e];
+  for (int i = t; i < kNint * kNl; i += kPmlThreads) {
+    tab[0][i] = tb.l[i / kNl][i % kNl];
+    tab[1][i] = tb.d[i / kNl][i % kNl];
+  }
   if (t < kNq) {
     const int q = t, intx = q % kNint, intz = q / kNint;
     QGeo g;
     if (!quad_geo(mv, dt, ie, q, true, g)) atomicCAS(err, 0, e + 1);
-    dcx ex = dcx{1.0, 0.0}, ez = dcx{1.0, 0.0};
+    PmlPoint w;
+    w.ex = w.ez = dcx{1.0, 0.0};
     if (g.xdep > 2.22e-16)
-      ex = zdampfn(g.xdep, g.vel, pp.xwidth, pp.dmax, logr, pp.kappa, pp.fcent, pp.omega);
+      w.ex = zdampfn(g.xdep, g.vel, pp.xwidth, pp.dmax, logr, pp.kappa, pp.fcent, pp.omega);
     if (g.zdep > 2.22e-16)
-      ez = zdampfn(g.zdep, g.vel, pp.zwidth, pp.dmax, logr, pp.kappa, pp.fcent, pp.omega);
-    double *c = qc + 11 * q;
-    c[0] = g.dxdxi; c[1] = g.dxdeta; c[2] = g.dzdxi; c[3] = g.dzdeta; c[4] = g.rjac;
-    double w = dt.wts[intx] * dt.wts[intz] * g.rjac;
-    c[5] = g.lam * w;
-    c[6] = g.mu * w;
-    c[7] = ex.re; c[8] = ex.im; c[9] = ez.re; c[10] = ez.im;
+      w.ez = zdampfn(g.zdep, g.vel, pp.zwidth, pp.dmax, logr, pp.kappa, pp.fcent, pp.omega);
+    w.x[0] = g.dzdeta / g.rjac;
+    w.x[1] = -g.dzdxi / g.rjac;
+    w.z[0] = -g.dxdeta / g.rjac;
+    w.z[1] = g.dxdxi / g.rjac;
+    const double f = dt.wts[intx] * dt.wts[intz] * g.rjac;
+    w.lam = g.lam * f;
+    w.mu = g.mu * f;
+    pt[q] = w;
   }
   __syncthreads();
-  for (int idx = t; idx < kNq * kNen; idx += kElemThreads) {
-    const int q = idx / kNen;
-    const double *c = qc + 11 * q;
-    const double *sl = dt.shl + 3 * (size_t)idx;
-    shx[idx] = (sl[0] * c[3] - sl[1] * c[2]) / c[4];
-    shz[idx] = -(sl[0] * c[1] - sl[1] * c[0]) / c[4];
-  }
-  __syncthreads();
-  if (t >= kNab) return;
-  const int a = t / kNen, b = t % kNen;
-  dcx acc[9];
+  double2 *out = pemat + (size_t)pe * kNab * 9;
+  for (int k = 3 * blockIdx.y; k < 3 * (int)blockIdx.y + 3; k++) {
+    const int bi = k / 3, bj = k % 3;
+    const bool ce1 = (bi + bj) & 1;
+    // kinds of CE0: (a, b) along (xi, xi), (xi, eta), (eta, xi), (eta, eta);
+    // of CE1: a along xi, a along eta, b along xi, b along eta
+    if (t < kNq) {
+      const PmlPoint w = pt[t];
+      const dcx xx = zmul(w.ex, w.ex), zz = zmul(w.ez, w.ez), xz = zmul(w.ex, w.ez);
+      const double c11 = w.lam + 2.0 * w.mu;
+      for (int kind = 0; kind < 4; kind++) {
+        const int s = kind >> 1, u = kind & 1;  // CE0: directions of a, b
+        dcx v;
+        if (!ce1) {
+          const double pxx = w.x[s] * w.x[u], pzz = w.z[s] * w.z[u];
+          const double pxz = w.x[s] * w.z[u], pzx = w.z[s] * w.x[u];
+          if (k == 0) v = zadd(zscale(c11 * pxx, xx), zscale(w.mu * pzz, zz));
+          else if (k == 4) v = zadd(zscale(w.mu * pxx, xx), zscale(w.mu * pzz, zz));
+          else if (k == 8) v = zadd(zscale(c11 * pzz, zz), zscale(w.mu * pxx, xx));
+          else if (k == 2) v = zscale(w.lam * pxz + w.mu * pzx, xz);
+          else v = zscale(w.lam * pzx + w.mu * pxz, xz);
+        } else {
+          // s: which of a (0) and b (1) is differentiated, u: its direction.
+          // (1,2) and (3,2): -(lambda d_a b - mu a d_b); (2,1) and (2,3):
+          // lambda a d_b - mu d_a b; along x with (1,2), (2,1), else along z
+          const bool first = k == 1 || k == 7, alongx = k == 1 || k == 3;
+          const double m = first ? (s == 0 ? -w.lam : w.mu) : (s == 0 ? -w.mu : w.lam);
+          v = alongx ? zscale(m * w.x[u], w.ex) : zscale(m * w.z[u], w.ez);
+        }
+        c[kind * kNq + t] = make_double2(v.re, v.im);
+      }
+    }
+    __syncthreads();
+    // which factors of a kind are derivatives: p, s of a and r, t of b
+    auto dp = [&](int kind) { return ce1 ? kind == 0 : kind < 2; };
+    auto dr = [&](int kind) { return ce1 ? kind == 2 : (kind & 1) == 0; };
+    auto ds = [&](int kind) { return ce1 ? kind == 1 : kind >= 2; };
+    auto dtt = [&](int kind) { return ce1 ? kind == 3 : (kind & 1) == 1; };
+    if (t < 4 * kNint * kNl) {
+      const int kind = t / (kNint * kNl), r = t % (kNint * kNl), qz = r / kNl, ix = r % kNl;
+      const double *P = tab[dp(kind)], *R = tab[dr(kind)];
+      const double2 *cq = c + kind * kNq + qz * kNint;
+      double2 a[kNl];
 #pragma unroll
-  for (int k = 0; k < 9; k++) acc[k] = dcx{0.0, 0.0};
-  for (int q = 0; q < kNq; q++) {
-    const double *c = qc + 11 * q;
-    const double lam = c[5], mu = c[6], c11 = lam + 2.0 * mu;
-    const dcx ex = dcx{c[7], c[8]}, ez = dcx{c[9], c[10]};
-    const double pa = dt.shl[3 * (q * kNen + a) + 2], pb = dt.shl[3 * (q * kNen + b) + 2];
-    const dcx pax = dcx{shx[q * kNen + a] * ex.re, shx[q * kNen + a] * ex.im};
-    const dcx paz = dcx{shz[q * kNen + a] * ez.re, shz[q * kNen + a] * ez.im};
-    const dcx pbx = dcx{shx[q * kNen + b] * ex.re, shx[q * kNen + b] * ex.im};
-    const dcx pbz = dcx{shz[q * kNen + b] * ez.re, shz[q * kNen + b] * ez.im};
-    // CE0 blocks
-    dcx xx = zmul(pax, pbx), zz = zmul(paz, pbz), xz = zmul(pax, pbz), zx = zmul(paz, pbx);
-    acc[0] = zadd(acc[0], dcx{c11 * xx.re + mu * zz.re, c11 * xx.im + mu * zz.im});
-    acc[2] = zadd(acc[2], dcx{lam * xz.re + mu * zx.re, lam * xz.im + mu * zx.im});
-    acc[4] = zadd(acc[4], dcx{mu * xx.re + mu * zz.re, mu * xx.im + mu * zz.im});
-    acc[6] = zadd(acc[6], dcx{lam * zx.re + mu * xz.re, lam * zx.im + mu * xz.im});
-    acc[8] = zadd(acc[8], dcx{c11 * zz.re + mu * xx.re, c11 * zz.im + mu * xx.im});
-    // CE1 blocks: i * (...)
-    dcx t12 = dcx{-(lam * pax.re * pb - mu * pa * pbx.re), -(lam * pax.im * pb - mu * pa * pbx.im)};
-    dcx t21 = dcx{lam * pa * pbx.re - mu * pax.re * pb, lam * pa * pbx.im - mu * pax.im * pb};
-    dcx t23 = dcx{lam * pa * pbz.re - mu * paz.re * pb, lam * pa * pbz.im - mu * paz.im * pb};
-    dcx t32 = dcx{-(lam * paz.re * pb - mu * pa * pbz.re), -(lam * paz.im * pb - mu * pa * pbz.im)};
-    acc[1] = zadd(acc[1], dcx{-t12.im, t12.re});
-    acc[3] = zadd(acc[3], dcx{-t21.im, t21.re});
-    acc[5] = zadd(acc[5], dcx{-t23.im, t23.re});
-    acc[7] = zadd(acc[7], dcx{-t32.im, t32.re});
-  }
-  double2 *o = pemat + ((size_t)pe * kNab + t) * 9;
+      for (int jx = 0; jx < kNl; jx++) a[jx] = make_double2(0.0, 0.0);
 #pragma unroll
-  for (int k = 0; k < 9; k++) o[k] = make_double2(acc[k].re, acc[k].im);
+      for (int qx = 0; qx < kNint; qx++) {
+        const double f = P[qx * kNl + ix];
+        const double2 v = make_double2(cq[qx].x * f, cq[qx].y * f);
+#pragma unroll
+        for (int jx = 0; jx < kNl; jx++) {
+          const double h = R[qx * kNl + jx];
+          a[jx].x += v.x * h;
+          a[jx].y += v.y * h;
+        }
+      }
+#pragma unroll
+      for (int jx = 0; jx < kNl; jx++) g[kind * kLine + (ix * kNl + jx) * kNint + qz] = a[jx];
+    }
+    __syncthreads();
+    const int hf = t / (kNl * kNen), u = t % (kNl * kNen);  // kinds {0, 1} or {2, 3}
+    const int ix = u % kNl, jx = (u / kNl) % kNl, iz = u / kNen;
+    double2 a[kNl];
+#pragma unroll
+    for (int jz = 0; jz < kNl; jz++) a[jz] = make_double2(0.0, 0.0);
+    if (hf < 2) {
+#pragma unroll
+      for (int o = 0; o < 2; o++) {
+        const int kind = 2 * hf + o;
+        const double *S = tab[ds(kind)], *T = tab[dtt(kind)];
+        const double2 *gl = g + kind * kLine + (ix * kNl + jx) * kNint;
+#pragma unroll
+        for (int qz = 0; qz < kNint; qz++) {
+          const double f = S[qz * kNl + iz];
+          const double2 v = make_double2(gl[qz].x * f, gl[qz].y * f);
+#pragma unroll
+          for (int jz = 0; jz < kNl; jz++) {
+            const double h = T[qz * kNl + jz];
+            a[jz].x += v.x * h;
+            a[jz].y += v.y * h;
+          }
+        }
+      }
+      if (hf == 1)
+#pragma unroll
+        for (int jz = 0; jz < kNl; jz++) half[u * kNl + jz] = a[jz];
+    }
+    __syncthreads();
+    if (hf == 0) {
+      const int na = ix + kNl * iz;
+#pragma unroll
+      for (int jz = 0; jz < kNl; jz++) {
+        const double2 b = half[u * kNl + jz];
+        const double re = a[jz].x + b.x, im = a[jz].y + b.y;
+        // CE1 carries the i of i omega py
+        out[(size_t)(na * kNen + jx + kNl * jz) * 9 + k] =
+            ce1 ? make_double2(-im, re) : make_double2(re, im);
+      }
+    }
+  }
+}
+
+static size_t pml_smem() {
+  return sizeof(double2) * (4 * kNq + 4 * kNl * kNl * kNint + kNab) + sizeof(PmlPoint) * kNq +
+         sizeof(double) * 2 * kNint * kNl;
 }
 
 // block id of element node pair (a,b): position of node B in block row A
@@ -741,8 +834,6 @@ __global__ void __launch_bounds__(T)
 // launchers
 // ---------------------------------------------------------------------------
 static size_t basis_smem() { return sizeof(double) * (3 * kNq * kNen + 8 * kNq); }
-static size_t pml_smem() { return sizeof(double) * (2 * kNq * kNen + 11 * kNq); }
-
 cudaError_t build_batch_structures(Ctx *c, cudaStream_t st) {
   cudaError_t e;
   const long long nb = c->bcsr.nblocks;
@@ -854,8 +945,8 @@ cudaError_t build_basis(Ctx *c, cudaStream_t st) {
 cudaError_t build_pml_delta(Ctx *c, const PmlParams &pp, int slot, cudaStream_t st) {
   if (c->npml_elem == 0 || c->npml_blocks == 0) return cudaSuccess;
   double logr = std::log(pp.rcoeff);
-  k_elem_pml<<<c->npml_elem, kElemThreads, pml_smem(), st>>>(c->mv, c->dt, c->d_pml_elems, pp, logr,
-                                                            c->d_pml_emat, c->d_err);
+  k_elem_pml<<<dim3(c->npml_elem, 3), kPmlThreads, pml_smem(), st>>>(
+      c->mv, c->dt, shape_tables(c->tab), c->d_pml_elems, pp, logr, c->d_pml_emat, c->d_err);
   long long npb = c->npml_blocks;
   k_gather_pml<<<(unsigned)((npb + 255) / 256), 256, 0, st>>>(
       npb, c->d_pgptr, c->d_pglist, c->d_pml_emat, c->d_pml_delta + (size_t)slot * npb * 9);
