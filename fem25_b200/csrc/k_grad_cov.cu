@@ -713,19 +713,35 @@ __global__ void k_cov_scale(const double2 *__restrict__ u, const double2 *__rest
 // Per element and combined block B (9 of them), with the shape functions
 // T_t(q)_(ix + 5 ie) = X_t(qx, ix) E_t(qz, ie) for t = N (X = l, E = l),
 // xi (l', l), eta (l, l'):
-//   Z_A[i][jx][qz]      = sum_je B[i][jx + 5 je] A(qz, je)                A = l, l'
-//   W_EA[ix][jx][qz]    = sum_ie E(qz, ie) Z_A[ix + 5 ie][jx][qz]        E = l, l'
+//   W_EA[ix][jx][qz]    = sum_ie E(qz, ie) sum_je A(qz, je) B[ix + 5 ie][jx + 5 je],  E, A = l, l'
 //   F^{t1 t2}(qz, qx)   = sum_jx X_t2(qx, jx) sum_ix X_t1(qx, ix) W_{E_t1 A_t2}[ix][jx][qz]
-// = T_t1(q)^T B T_t2(q): about 0.28 M FMA per element.
+// = T_t1(q)^T B T_t2(q): about 0.3 M FMA per element.
+// Bound: the latency of its chains and the shared-memory reads beside them (75 KB
+// of blocks an element from HBM would take 0.5 ms for 43 600 elements, the operations
+// 0.7).  A thread serves two mirrored points of each step (l_i(-x) = l_{4-i}(x)), so
+// that a value read feeds two; three blocks are in work at once, with the next three's
+// raw blocks on their way by cp.async, and the metric is made once per element:
+// 31 000 warp instructions an element and 10 barriers.  43 600 elements: 3.09 ms
+// against 3.45 with one block at a time through a separate first step in shared
+// memory (28 barriers).  A warp per combined block with the W's of a line in registers
+// read a tenth as much shared memory but left two warps a scheduler: 4.26 ms.
 namespace covf {
-constexpr int kThreads = 256;
+constexpr int kThreads = 288;
+constexpr int kHalf = kNint / 2 + 1;         // 7 points and their mirrors
 constexpr int kRawMax = 3;                   // raw blocks behind one combined block
-constexpr int kRaw = kRawMax * cov::kBlk;    // doubles per raw buffer
-constexpr int kZ = kNen * kNl * kNint;       // 1625: Z[i][jx][qz]
+constexpr int kGroupRaw = 6;                 // raw blocks of a group of three
 constexpr int kW = kNl * kNl * kNint;        // 325: W[ix][jx][qz]
-constexpr int kSmemDoubles = 2 * kRaw + 2 * kZ + 4 * kW + 2 * kNint * kNl + 4 * kNq;
-constexpr int kSmemBytes = kSmemDoubles * 8;  // 72 KB: three CTAs per SM
+constexpr int kWMax = 10;                    // W's of a group
+constexpr int kSmemDoubles =
+    kGroupRaw * cov::kBlk + 3 * kNen * kNen + kWMax * kW + 5 * kNq;
+constexpr int kSmemBytes = kSmemDoubles * 8;  // 78 KB
 }  // namespace covf
+
+// Group g works on the combined blocks 3 g + slot (equal numbers of forms): their
+// first raw block in the group's buffer and their first W.  Blocks 0-2 take W_ll,
+// W_ld, W_dd (B is symmetric), block 3 all four, 4 and 5 W_ll, W_ld, W_dl, 6-8 W_ll.
+__device__ constexpr int kCovRaw0[3][3] = {{0, 1, 2}, {0, 2, 4}, {0, 1, 3}};
+__device__ constexpr int kCovW0[3][3] = {{0, 3, 6}, {0, 4, 7}, {0, 1, 2}};
 
 // raw blocks behind combined block b (stored [j][i]): first index and count
 __device__ __forceinline__ void cov_raw_of(int b, int *ids, int &n) {
@@ -755,207 +771,293 @@ __device__ __forceinline__ double cov_bval(int b, const double *r, int i, int j)
   }
 }
 
-// sum_jx x2[jx] sum_ix x1[ix] W[ix][jx][qz]
-__device__ __forceinline__ double cov_fw(const double *W, int qz, const double *x1,
-                                         const double *x2) {
-  double f = 0.0;
+// 1D factors of a point x and, by symmetry, of its mirror
+struct CovPt {
+  double l[kNl], d[kNl];
+};
+
+// sum_jx X2[jx] sum_ix X1[ix] W[ix][jx][qz] at a point (a) and its mirror (b),
+// X = l or (D) l'
+template <bool D1, bool D2>
+__device__ __forceinline__ void cov_fw(const double *W, const CovPt &x, double &a, double &b) {
+  a = 0.0;
+  b = 0.0;
 #pragma unroll
   for (int jx = 0; jx < kNl; jx++) {
-    double h = 0.0;
+    double ha = 0.0, hb = 0.0;
 #pragma unroll
-    for (int ix = 0; ix < kNl; ix++) h = fma(x1[ix], W[(ix * kNl + jx) * kNint + qz], h);
-    f = fma(x2[jx], h, f);
+    for (int ix = 0; ix < kNl; ix++) {
+      const double w = W[(ix * kNl + jx) * kNint];
+      ha = fma(D1 ? x.d[ix] : x.l[ix], w, ha);
+      hb = fma(D1 ? x.d[kNl - 1 - ix] : x.l[kNl - 1 - ix], w, hb);
+    }
+    a = fma(D2 ? x.d[jx] : x.l[jx], ha, a);
+    b = fma(D2 ? x.d[kNl - 1 - jx] : x.l[kNl - 1 - jx], hb, b);
   }
-  return f;
+  if (D1 != D2) b = -b;  // l' changes sign at the mirror
 }
 
-__global__ void __launch_bounds__(covf::kThreads, 3)
+__global__ void __launch_bounds__(covf::kThreads, 2)
     k_grad_cov_fin(MeshView mv, DevTables dt, int n_elem, int nnpg, const int *__restrict__ elems,
                    const double *__restrict__ accb, ShapeTabs tb, double *__restrict__ grad,
                    int *__restrict__ err) {
   extern __shared__ __align__(16) double fs[];
-  double *rawb = fs;                          // [2][kRaw]
-  double *zl = rawb + 2 * covf::kRaw, *zd = zl + covf::kZ;
-  double *wb = zd + covf::kZ;                 // [4][kW]: (E, A) = (l,l) (l,l') (l',l) (l',l')
-  double *tl_s = wb + 4 * covf::kW, *td_s = tl_s + kNint * kNl;  // 1D tables
-  double *wsf_s = td_s + kNint * kNl;         // [4][169] W_q SF_a(q)
+  double *raw = fs;                                 // [kGroupRaw][kBlk]
+  double *wb = raw + covf::kGroupRaw * cov::kBlk;   // [kWMax][kW]
+  double *bb = wb + covf::kWMax * covf::kW;         // [3][25][25] B[i][j] at j * 25 + i
+  double *geo = bb + 3 * kNen * kNen;               // [5][169]: ax, bx, az, bz, weight
   __shared__ double red[12][covf::kThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int k = tid; k < kNint * kNl; k += covf::kThreads) {
-    tl_s[k] = tb.l[k / kNl][k % kNl];
-    td_s[k] = tb.d[k / kNl][k % kNl];
+  // combined blocks: column i of 25, rows 11 apart
+  const int ci = tid % kNen, cj = tid / kNen;
+  // W stage: 7 points z, a thread keeps its own; (block, ix, jx) 41 apart
+  constexpr int kWStep = covf::kThreads / covf::kHalf;
+  const int wz = tid % covf::kHalf, wu = tid / covf::kHalf;
+  double l[kNl], d[kNl];
+#pragma unroll
+  for (int i = 0; i < kNl; i++) {
+    l[i] = tb.l[wz][i];
+    d[i] = tb.d[wz][i];
   }
-  const bool ptq = tid < kNq;
-  const int q = ptq ? tid : 0, qx = q % kNint, qz = q / kNint;
+  // F stage: block slot of the group, point (qx, qz) and its mirror in xi
+  constexpr int kPts = covf::kHalf * kNint;
+  const bool pts = tid < 3 * kPts;
+  const int slot = pts ? tid / kPts : 0, pp = pts ? tid % kPts : 0;
+  const int qx = pp % covf::kHalf, qz = pp / covf::kHalf;
+  const int qa = qx + kNint * qz, qb = kNint - 1 - qx + kNint * qz;
+  CovPt x;
+#pragma unroll
+  for (int i = 0; i < kNl; i++) {
+    x.l[i] = tb.l[qx][i];
+    x.d[i] = tb.d[qx][i];
+  }
   const int my_elems = (n_elem - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int ntask = max(my_elems, 0) * 9;     // tasks (element, combined block)
+  const int ntask = max(my_elems, 0) * 3;  // tasks (element, group)
 
-  // copies the raw blocks of task k into raw buffer k & 1 (16-byte cp.async)
+  // copies the raw blocks of task k to shared memory (16-byte cp.async)
   auto fetch = [&](int k) {
     if (k < ntask) {
-      const int ei = (int)blockIdx.x + (k / 9) * (int)gridDim.x, b = k % 9;
-      int ids[covf::kRawMax], n;
-      cov_raw_of(b, ids, n);
-      double *dst = rawb + (k & 1) * covf::kRaw;
+      const int ei = (int)blockIdx.x + (k / 3) * (int)gridDim.x, g = k % 3;
       const double *src = accb + (size_t)ei * cov::kBlocks * cov::kBlk;
       constexpr int kV = cov::kBlk / 2;  // 16-byte vectors per block
-      for (int v = tid; v < n * kV; v += covf::kThreads) {
-        const int r = v / kV, o = 2 * (v % kV);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + r * cov::kBlk + o)),
-                     "l"(src + (size_t)ids[r] * cov::kBlk + o)
-                     : "memory");
+#pragma unroll
+      for (int s = 0; s < 3; s++) {
+        int ids[covf::kRawMax], n;
+        cov_raw_of(3 * g + s, ids, n);
+        for (int r = 0; r < n; r++) {
+          const double *from = src + (size_t)ids[r] * cov::kBlk;
+          const unsigned to = smem_u32(raw + (kCovRaw0[g][s] + r) * cov::kBlk);
+          for (int v = tid; v < kV; v += covf::kThreads)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16 * v),
+                         "l"(from + 2 * v)
+                         : "memory");
+        }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  double ax = 0.0, bx = 0.0, az = 0.0, bz = 0.0;  // inverse Jacobian rows at point q
-  double xl[kNl], xd[kNl];                         // l(qx, .), l'(qx, .)
-  double tl = 0.0, tm = 0.0, tr = 0.0;
+  double tl[2], tm[2], tr[2];
   fetch(0);
   for (int k = 0; k < ntask; k++) {
-    const int ei = (int)blockIdx.x + (k / 9) * (int)gridDim.x, b = k % 9;
+    const int ei = (int)blockIdx.x + (k / 3) * (int)gridDim.x, g = k % 3;
     const int4 ie = mv.ieng[elems[ei]];
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // task k's raw blocks visible; task k - 1 done with every buffer
+    __syncthreads();  // task k's raw blocks visible
+    // ---- the group's combined blocks
+    if (cj < covf::kThreads / kNen)
+#pragma unroll
+      for (int s = 0; s < 3; s++) {
+        const double *r = raw + kCovRaw0[g][s] * cov::kBlk;
+        for (int j = cj; j < kNen; j += covf::kThreads / kNen)
+          bb[s * kNen * kNen + j * kNen + ci] = cov_bval(3 * g + s, r, ci, j);
+      }
+    __syncthreads();  // and every thread is past task k - 1's W's and metric
     fetch(k + 1);
-    if (b == 0) {
-      if (k == 0) {
+    if (g == 0 && tid < kNq) {  // inverse Jacobian rows and weights at the points
+      QGeo q;
+      if (!quad_geo(mv, dt, ie, tid, false, q)) atomicCAS(err, 0, elems[ei] + 1);
+      const double rj = 1.0 / q.rjac;
+      geo[tid] = q.dzdeta * rj;
+      geo[kNq + tid] = -q.dzdxi * rj;
+      geo[2 * kNq + tid] = -q.dxdeta * rj;
+      geo[3 * kNq + tid] = q.dxdxi * rj;
+      geo[4 * kNq + tid] = dt.wts[tid % kNint] * dt.wts[tid / kNint] * q.rjac;
+    }
+    // ---- W stage: task (block, ix, jx) at the points wz and 12 - wz
+    for (int t = wu; wu < kWStep && t < 3 * kNl * kNl; t += kWStep) {
+      const int s = t / (kNl * kNl), ij = t - s * kNl * kNl, ix = ij / kNl, jx = ij - ix * kNl;
+      const int b = 3 * g + s;
+      const double *Bs = bb + s * kNen * kNen + jx * kNen + ix;
+      double *wo = wb + kCovW0[g][s] * covf::kW + ij * kNint + wz, *wm = wo + kNint - 1 - 2 * wz;
+      // [point, mirror] of W_ll, W_ld, W_dl, W_dd
+      double ll[2] = {0.0, 0.0}, ld[2] = {0.0, 0.0}, dl[2] = {0.0, 0.0}, dd[2] = {0.0, 0.0};
+      if (b >= 6) {
 #pragma unroll
         for (int i = 0; i < kNl; i++) {
-          xl[i] = tl_s[qx * kNl + i];
-          xd[i] = td_s[qx * kNl + i];
+          double sa = 0.0, sb = 0.0;
+#pragma unroll
+          for (int j = 0; j < kNl; j++) {
+            const double v = Bs[j * kNl * kNen + i * kNl];
+            sa = fma(l[j], v, sa);
+            sb = fma(l[kNl - 1 - j], v, sb);
+          }
+          ll[0] = fma(l[i], sa, ll[0]);
+          ll[1] = fma(l[kNl - 1 - i], sb, ll[1]);
         }
+        wo[0] = ll[0];
+        wm[0] = ll[1];
+        continue;
       }
-      tl = tm = tr = 0.0;
-      if (ptq) {
-        QGeo g;
-        if (!quad_geo(mv, dt, ie, q, false, g)) atomicCAS(err, 0, elems[ei] + 1);
-        ax = g.dzdeta / g.rjac;
-        bx = -g.dzdxi / g.rjac;
-        az = -g.dxdeta / g.rjac;
-        bz = g.dxdxi / g.rjac;
-        const double wq = dt.wts[qx] * dt.wts[qz] * g.rjac;
 #pragma unroll
-        for (int a = 0; a < 4; a++) wsf_s[a * kNq + q] = dt.sf[4 * q + a] * wq;
-      }
-    }
-    const double *r = rawb + (k & 1) * covf::kRaw;
-    const bool two = b < 6;  // Z_l' and the W's beyond (l, l) needed
-    // ---- Z stage: task (i, jx)
-    if (tid < kNen * kNl) {
-      const int i = tid / kNl, jx = tid % kNl;
-      double bv[kNl];
+      for (int i = 0; i < kNl; i++) {
+        double sa = 0.0, sb = 0.0, ta = 0.0, tc = 0.0;  // l and l' sums; tc: -l' at the mirror
 #pragma unroll
-      for (int je = 0; je < kNl; je++) bv[je] = cov_bval(b, r, i, jx + kNl * je);
-      double *ol = zl + (i * kNl + jx) * kNint, *od = zd + (i * kNl + jx) * kNint;
-#pragma unroll
-      for (int z = 0; z < kNint; z++) {
-        double sl = 0.0, sd = 0.0;
-#pragma unroll
-        for (int je = 0; je < kNl; je++) {
-          sl = fma(bv[je], tb.l[z][je], sl);
-          sd = fma(bv[je], tb.d[z][je], sd);
+        for (int j = 0; j < kNl; j++) {
+          const double v = Bs[j * kNl * kNen + i * kNl];
+          sa = fma(l[j], v, sa);
+          sb = fma(l[kNl - 1 - j], v, sb);
+          ta = fma(d[j], v, ta);
+          tc = fma(d[kNl - 1 - j], v, tc);
         }
-        ol[z] = sl;
-        if (two) od[z] = sd;
+        ll[0] = fma(l[i], sa, ll[0]);
+        ll[1] = fma(l[kNl - 1 - i], sb, ll[1]);
+        ld[0] = fma(l[i], ta, ld[0]);
+        ld[1] = fma(l[kNl - 1 - i], tc, ld[1]);
+        dl[0] = fma(d[i], sa, dl[0]);
+        dl[1] = fma(d[kNl - 1 - i], sb, dl[1]);
+        dd[0] = fma(d[i], ta, dd[0]);
+        dd[1] = fma(d[kNl - 1 - i], tc, dd[1]);
       }
-    }
-    __syncthreads();
-    // ---- W stage: task (ix, jx, qz)
-    for (int t = tid; t < covf::kW; t += covf::kThreads) {
-      const int z = t % kNint, ixjx = t / kNint, ix = ixjx / kNl, jx = ixjx % kNl;
-      double w0 = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0;
-#pragma unroll
-      for (int ie2 = 0; ie2 < kNl; ie2++) {
-        const int zi = ((ix + kNl * ie2) * kNl + jx) * kNint + z;
-        const double a = zl[zi];
-        const double el = tl_s[z * kNl + ie2], ed = td_s[z * kNl + ie2];
-        w0 = fma(el, a, w0);
-        if (two) {
-          const double c = zd[zi];
-          w1 = fma(el, c, w1);
-          w2 = fma(ed, a, w2);
-          w3 = fma(ed, c, w3);
-        }
-      }
-      wb[t] = w0;
-      if (two) {
-        wb[covf::kW + t] = w1;
-        wb[2 * covf::kW + t] = w2;
-        wb[3 * covf::kW + t] = w3;
+      wo[0] = ll[0];
+      wm[0] = ll[1];
+      wo[covf::kW] = ld[0];
+      wm[covf::kW] = -ld[1];
+      // blocks 0-2: W_dd; 4, 5: W_dl; 3: both
+      wo[2 * covf::kW] = b < 3 ? dd[0] : dl[0];
+      wm[2 * covf::kW] = b < 3 ? dd[1] : -dl[1];
+      if (b == 3) {
+        wo[3 * covf::kW] = dd[0];
+        wm[3 * covf::kW] = dd[1];
       }
     }
     __syncthreads();
-    // ---- F stage: point q
-    if (ptq) {
-      const double *W0 = wb, *W1 = wb + covf::kW, *W2 = wb + 2 * covf::kW, *W3 = wb + 3 * covf::kW;
+    // ---- F stage: the forms of one block at two points
+    if (g == 0) tl[0] = tl[1] = tm[0] = tm[1] = tr[0] = tr[1] = 0.0;
+    if (pts) {
+      const int b = 3 * g + slot;
+      const double ax[2] = {geo[qa], geo[qb]}, bx[2] = {geo[kNq + qa], geo[kNq + qb]};
+      const double az[2] = {geo[2 * kNq + qa], geo[2 * kNq + qb]};
+      const double bz[2] = {geo[3 * kNq + qa], geo[3 * kNq + qb]};
+      const double *W0 = wb + kCovW0[g][slot] * covf::kW + qz;
+      const double *W1 = W0 + covf::kW, *W2 = W1 + covf::kW, *W3 = W2 + covf::kW;
+      double f[4][2];
       if (b < 3) {
-        const double fxx = cov_fw(W0, qz, xd, xd), fxe = cov_fw(W1, qz, xd, xl);
-        const double fee = cov_fw(W3, qz, xl, xl);
-        const double xx = ax * ax * fxx + 2.0 * ax * bx * fxe + bx * bx * fee;
-        const double zz = az * az * fxx + 2.0 * az * bz * fxe + bz * bz * fee;
-        if (b == 0) {
-          tl += xx;
-          tm += 2.0 * xx + zz;
-        } else if (b == 1) {
-          tl += zz;
-          tm += xx + 2.0 * zz;
-        } else {
-          tm += xx + zz;
+        cov_fw<true, true>(W0, x, f[0][0], f[0][1]);    // xi, xi
+        cov_fw<true, false>(W1, x, f[1][0], f[1][1]);   // xi, eta
+        cov_fw<false, false>(W2, x, f[2][0], f[2][1]);  // eta, eta
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const double xx = ax[h] * ax[h] * f[0][h] + 2.0 * ax[h] * bx[h] * f[1][h] + bx[h] * bx[h] * f[2][h];
+          const double zz = az[h] * az[h] * f[0][h] + 2.0 * az[h] * bz[h] * f[1][h] + bz[h] * bz[h] * f[2][h];
+          if (b == 0) {
+            tl[h] += xx;
+            tm[h] += 2.0 * xx + zz;
+          } else if (b == 1) {
+            tl[h] += zz;
+            tm[h] += xx + 2.0 * zz;
+          } else {
+            tm[h] += xx + zz;
+          }
         }
       } else if (b == 3) {
-        const double fxx = cov_fw(W0, qz, xd, xd), fxe = cov_fw(W1, qz, xd, xl);
-        const double fex = cov_fw(W2, qz, xl, xd), fee = cov_fw(W3, qz, xl, xl);
-        tl += ax * az * fxx + ax * bz * fxe + bx * az * fex + bx * bz * fee;  // x^T S z
-        tm += az * ax * fxx + az * bx * fxe + bz * ax * fex + bz * bx * fee;  // z^T S x
+        cov_fw<true, true>(W0, x, f[0][0], f[0][1]);
+        cov_fw<true, false>(W1, x, f[1][0], f[1][1]);
+        cov_fw<false, true>(W2, x, f[2][0], f[2][1]);
+        cov_fw<false, false>(W3, x, f[3][0], f[3][1]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          tl[h] += ax[h] * az[h] * f[0][h] + ax[h] * bz[h] * f[1][h] + bx[h] * az[h] * f[2][h] +
+                   bx[h] * bz[h] * f[3][h];  // x^T S z
+          tm[h] += az[h] * ax[h] * f[0][h] + az[h] * bx[h] * f[1][h] + bz[h] * ax[h] * f[2][h] +
+                   bz[h] * bx[h] * f[3][h];  // z^T S x
+        }
       } else if (b < 6) {
-        const double fxn = cov_fw(W0, qz, xd, xl), fen = cov_fw(W2, qz, xl, xl);
-        const double fnx = cov_fw(W0, qz, xl, xd), fne = cov_fw(W1, qz, xl, xl);
-        if (b == 4) {
-          tl += ax * fxn + bx * fen;  // x^T G1 v
-          tm -= ax * fnx + bx * fne;  // v^T G1 x
-        } else {
-          tl += az * fxn + bz * fen;  // z^T G2 v
-          tm -= az * fnx + bz * fne;  // v^T G2 z
+        cov_fw<true, false>(W0, x, f[0][0], f[0][1]);   // xi, N
+        cov_fw<false, false>(W2, x, f[1][0], f[1][1]);  // eta, N
+        cov_fw<false, true>(W0, x, f[2][0], f[2][1]);   // N, xi
+        cov_fw<false, false>(W1, x, f[3][0], f[3][1]);  // N, eta
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const double p = b == 4 ? ax[h] : az[h], q = b == 4 ? bx[h] : bz[h];
+          tl[h] += p * f[0][h] + q * f[1][h];  // x^T G1 v, z^T G2 v
+          tm[h] -= p * f[2][h] + q * f[3][h];  // v^T G1 x, v^T G2 z
         }
       } else {
-        const double fnn = cov_fw(W0, qz, xl, xl);
-        if (b == 6) {
-          tl += fnn;
-          tm += 2.0 * fnn;
-        } else if (b == 7) {
-          tm += fnn;
-        } else {
-          tr -= fnn;
+        cov_fw<false, false>(W0, x, f[0][0], f[0][1]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          if (b == 6) {
+            tl[h] += f[0][h];
+            tm[h] += 2.0 * f[0][h];
+          } else if (b == 7) {
+            tm[h] += f[0][h];
+          } else {
+            tr[h] -= f[0][h];
+          }
         }
       }
     }
-    if (b == 8) {
-      // ---- g_{m, anchor a} += sum_q W_q SF_a(q) T_m(q)
-      double v[12];
+    if (g == 2) {
+      // ---- g_{m, anchor a} += sum_q W_q SF_a(q) T_m(q); the mirror of the middle
+      // column is the point itself
+      // sums of the three slots' parts, through the spent W's
+      __syncthreads();
+      if (pts && slot > 0)
 #pragma unroll
-      for (int a = 0; a < 4; a++) {
-        const double w = ptq ? wsf_s[a * kNq + q] : 0.0;
-        v[3 * a + 0] = w * tl;
-        v[3 * a + 1] = w * tm;
-        v[3 * a + 2] = w * tr;
-      }
+        for (int h = 0; h < 2; h++) {
+          double *o = wb + ((slot - 1) * 6 + 3 * h) * kPts + pp;
+          o[0] = tl[h];
+          o[kPts] = tm[h];
+          o[2 * kPts] = tr[h];
+        }
+      __syncthreads();
+      if (warp < (kPts + 31) / 32) {
+        double v[12];
 #pragma unroll
-      for (int kk = 0; kk < 12; kk++) {
-        double x = v[kk];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        v[kk] = x;
+        for (int m = 0; m < 12; m++) v[m] = 0.0;
+        if (tid < kPts) {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            if (h == 1 && qa == qb) break;
+            const double *o = wb + 3 * h * kPts + pp, *o2 = o + 6 * kPts;
+            const double sl = tl[h] + o[0] + o2[0], sm = tm[h] + o[kPts] + o2[kPts],
+                         sr = tr[h] + o[2 * kPts] + o2[2 * kPts];
+            const int q = h ? qb : qa;
+            const double wq = geo[4 * kNq + q];
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+              const double w = dt.sf[4 * q + a] * wq;
+              v[3 * a + 0] += w * sl;
+              v[3 * a + 1] += w * sm;
+              v[3 * a + 2] += w * sr;
+            }
+          }
+        }
+#pragma unroll
+        for (int kk = 0; kk < 12; kk++) {
+          double y = v[kk];
+          for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+          if (lane == 0) red[kk][warp] = y;
+        }
       }
-      if (lane == 0)
-        for (int kk = 0; kk < 12; kk++) red[kk][warp] = v[kk];
       __syncthreads();
       if (tid < 12) {
-        double x = 0.0;
-        for (int w = 0; w < covf::kThreads / 32; w++) x += red[tid][w];
+        double y = 0.0;
+        for (int w = 0; w < (kPts + 31) / 32; w++) y += red[tid][w];
         const int a = tid / 3, m = tid % 3;
         const int anchor = (a == 0 ? ie.x : a == 1 ? ie.y : a == 2 ? ie.z : ie.w) - 1;
-        atomicAdd(&grad[(size_t)m * nnpg + anchor], x);
+        atomicAdd(&grad[(size_t)m * nnpg + anchor], y);
       }
     }
   }
@@ -1166,7 +1268,7 @@ cudaError_t launch_grad_cov_fin(Ctx *c, double *grad, cudaStream_t st) {
   if (!c->cov_pending || c->n_nonpml == 0) return cudaSuccess;
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-  const int grid = std::min(3 * nsm, c->n_nonpml);
+  const int grid = std::min(2 * nsm, c->n_nonpml);
   k_grad_cov_fin<<<grid, covf::kThreads, covf::kSmemBytes, st>>>(
       c->mv, c->dt, c->n_nonpml, c->nnpg, c->d_nonpml, c->d_cov, shape_tables(c->tab), grad,
       c->d_err);
