@@ -26,12 +26,13 @@ namespace fem25 {
 namespace {
 
 constexpr int kPanelThreads = 512;
+constexpr int kSmThreads = 256, kSmRows = 390, kSmLd = kSmRows + 1;  // panel in shared memory
 constexpr int kLuThreads = 256;
 constexpr int kLuRows = 128;     // threads of k_sp_lu that hold a row of a sub-panel
 constexpr int kTrsmThreads = 128, kStrip = 32;
-constexpr int kGemmThreads = 128, kTile = 64, kKc = 8;
-constexpr int kGemmLda = kTile + 2, kGemmLdb = kKc + 4;  // conflict-free fragment reads
-constexpr int kGemmStage = kKc * kGemmLda + kTile * kGemmLdb;  // double2 per stage
+constexpr int kGemmThreads = 128, kTile = 64, kGt = 32, kKc = 8;
+constexpr int kGemmLda = kGt + 2, kGemmLdb = kKc + 4;  // conflict-free fragment reads
+constexpr int kGemmStage = kKc * kGemmLda + kGt * kGemmLdb;  // double2 per stage
 
 // ---------------------------------------------------------------------------
 // assembly of a level's fronts
@@ -93,13 +94,20 @@ __global__ void k_sp_entries(long long n, const int *__restrict__ idx,
 template <int W, int NW>
 struct PanelShared {
   unsigned key[2][NW];
-  int idx[2][NW];
   double2 prow[2][W], jrow[2][W];
   int swap[W];
 };
 
-// Pivot size |re| + |im| to 20 bits: the upper word of a non-negative double
-// orders like it; NaN counts as 0
+// Candidate row r < 4096 of a pivot search as one word: the size |re| + |im| to 9
+// bits after the leading one (the upper word of a non-negative double orders like
+// it; NaN counts as 0), then the lowest row first.  A pivot is thus at least 0.998 of
+// the column's largest entry.
+__device__ __forceinline__ unsigned pivot_word(double2 v, int r) {
+  const double a = fabs(v.x) + fabs(v.y);
+  const unsigned key = a >= 0.0 ? (unsigned)__double2hiint(a) : 0u;
+  return (key << 1 & ~0xfffu) | (unsigned)(4095 - r);
+}
+// the same without a row, to 20 bits
 __device__ __forceinline__ unsigned pivot_key(double2 v) {
   const double a = fabs(v.x) + fabs(v.y);
   return a >= 0.0 ? (unsigned)__double2hiint(a) : 0u;
@@ -113,43 +121,37 @@ __device__ __forceinline__ void bar_rows() {
   asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
 }
 
+// 1 / v, zero when v is no pivot
+__device__ __forceinline__ double2 crecip(double2 v) {
+  if (!pivot_ok(v)) return make_double2(0.0, 0.0);
+  const double d = 1.0 / (v.x * v.x + v.y * v.y);
+  return make_double2(v.x * d, -v.y * d);
+}
+
 // LU with partial pivoting of the w <= W columns a[q][0..w) of rows
 // r = t + q T < nrow; thread t keeps position r, interchanges move the contents.
-// The pivot is the row of largest |re| + |im| to 20 bits (the upper word of the
-// double), the lowest such row among equals.  s.swap[j] = row interchanged with
-// j.  Returns true when a pivot was zero (or NaN).  Two barriers a column.
+// s.swap[j] = row interchanged with j.  Returns true when a pivot was zero (or NaN).
+// Two barriers a column.
 template <int W, int RPT, int T>
 __device__ __forceinline__ bool lu_columns(double2 (&a)[RPT][W], int w, int nrow, int t,
                                            PanelShared<W, T / 32> &s) {
+  static_assert(RPT * T <= 4096, "pivot_word holds 12 bits of row");
   const int lane = t & 31, warp = t >> 5;
   bool zero = false;
 #pragma unroll
   for (int j = 0; j < W; j++) {
     if (j < w) {
       unsigned best = 0;
-      int bi = INT_MAX;
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
         const int r = t + q * T;
-        if (r >= j && r < nrow) {
-          const unsigned key = pivot_key(a[q][j]);
-          if (bi == INT_MAX || key > best) {
-            best = key;
-            bi = r;
-          }
-        }
+        if (r >= j && r < nrow) best = max(best, pivot_word(a[q][j], r));
       }
       const unsigned wm = __reduce_max_sync(0xffffffffu, best);
-      const int wi = __reduce_min_sync(0xffffffffu, best == wm ? bi : INT_MAX);
-      if (lane == 0) {
-        s.key[j & 1][warp] = wm;
-        s.idx[j & 1][warp] = wi;
-      }
+      if (lane == 0) s.key[j & 1][warp] = wm;
       bar_rows<T>();
-      const unsigned ck = lane < T / 32 ? s.key[j & 1][lane] : 0u;
-      const int ci = lane < T / 32 ? s.idx[j & 1][lane] : INT_MAX;
-      const unsigned bm = __reduce_max_sync(0xffffffffu, ci == INT_MAX ? 0u : ck);
-      const int p = __reduce_min_sync(0xffffffffu, ck == bm ? ci : INT_MAX);
+      const unsigned bm = __reduce_max_sync(0xffffffffu, lane < T / 32 ? s.key[j & 1][lane] : 0u);
+      const int p = 4095 - (int)(bm & 0xfffu);
       if (t == 0) s.swap[j] = p;
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
@@ -167,7 +169,7 @@ __device__ __forceinline__ bool lu_columns(double2 (&a)[RPT][W], int w, int nrow
       for (int c = j; c < W; c++) u[c] = s.prow[j & 1][c];
       const bool z = !pivot_ok(u[j]);
       zero |= z;
-      const double2 inv = z ? make_double2(0.0, 0.0) : cdiv(make_double2(1.0, 0.0), u[j]);
+      const double2 inv = crecip(u[j]);
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
         const int r = t + q * T;
@@ -211,7 +213,7 @@ __device__ __forceinline__ void invert_triangle(double2 *D, int ld, int nb, int 
     for (int i = g; i < nb; i += gt) {
       if (up) {
         const double2 d = D[i + i * ld];
-        dinv[i] = pivot_ok(d) ? cdiv(make_double2(1.0, 0.0), d) : make_double2(0.0, 0.0);
+        dinv[i] = crecip(d);
       } else {
         buf[0][i] = D[i];
       }
@@ -391,15 +393,19 @@ __global__ void __launch_bounds__(kLuThreads)
 
 // The triangular solves of a small front, strips of 32: blockIdx.y below the
 // front's count of column strips: U12 = L11^-1 P F12 of 32 boundary columns;
-// then row strips of L21 = F21 U11^-1.  A warp owns 8 columns (rows) of its
-// strip, so only the staged block of L (U) is shared: per block of 32 the
-// product with the inverted diagonal block, then the update of the rows
-// (columns) still to come, as 8 x 8 tensor-core tiles.
+// then row strips of L21 = F21 U11^-1.  A warp owns 8 columns (rows) of its strip,
+// so that warps never wait for one another: per block of 32 the product with the
+// inverted diagonal block, then the update of the rows (columns) still to come, as
+// 8 x 8 tensor-core tiles whose factor operand is loaded straight from the store
+// (16 loads in flight a lane).  Staging it in shared memory cost two CTA barriers a
+// block and left two CTAs an SM: 4.8 ms over all levels against 4.4.
+// Rows and columns past k read the last ones instead; they meet zeros, or their
+// results are not kept.
 __global__ void __launch_bounds__(kTrsmThreads)
     k_sp_trsm(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
               const double2 *__restrict__ work, double2 *__restrict__ fac,
               const int *__restrict__ perm) {
-  extern __shared__ double2 sh[];
+  extern __shared__ double2 X[];
   const SpFront f = fr[fronts[blockIdx.x]];
   const int k = f.k, m = f.m, n = k + m;
   const int nstrip = (m + kStrip - 1) / kStrip;
@@ -407,48 +413,29 @@ __global__ void __launch_bounds__(kTrsmThreads)
   const bool rows = (int)blockIdx.y >= nstrip;  // L21
   const int s0 = ((int)blockIdx.y - (rows ? nstrip : 0)) * kStrip, ns = min(kStrip, m - s0);
   const int kp = (k + 7) & ~7;
-  const int ldx = rows ? kStrip + 2 : kp + 5;   // X[strip row][k] or X[k][strip column]
-  const int ldt = rows ? sp::kNb + 4 : kp + 2;  // T = U(block, :) or L(:, block)
-  double2 *X = sh, *T = sh + (rows ? (kStrip + 2) * kp : (kp + 5) * kStrip);
+  const int ldx = rows ? kStrip + 2 : kp + 5;  // X[strip row][k] or X[k][strip column]
   const double2 *F = work + f.work0;
   double2 *L = fac + f.fac0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int lr = lane >> 2, lk = lane & 3;
   constexpr int nw = kTrsmThreads / 32;
-  const double2 zero = make_double2(0.0, 0.0);
+  const double2 zero = make_double2(0.0, 0.0), one = make_double2(1.0, 0.0);
   if (!rows) {
-    for (int c = warp; c < kStrip; c += nw)
+    for (int c = 8 * warp; c < 8 * warp + 8; c++)
       for (int r = lane; r < kp; r += 32)
         X[r + c * ldx] = (c < ns && r < k)
                              ? F[perm[f.own0 + r] + (long long)(k + s0 + c) * n] : zero;
+    __syncwarp();
   } else {
     for (int c = warp; c < kp; c += nw)
       X[lane + c * ldx] = (lane < ns && c < k) ? F[k + s0 + lane + (long long)c * n] : zero;
+    __syncthreads();
   }
+  auto at = [&](int r, int c) {
+    return L[min(r, k - 1) + (long long)min(c, k - 1) * n];
+  };
   for (int jb = 0; jb < k; jb += sp::kNb) {
-    const int nb = min(sp::kNb, k - jb), rest = kp - jb;  // rest: from the block on, padded
-    __syncthreads();
-    // T: the block column of L (rows jb..) or block row of U (columns jb..), the
-    // diagonal block with its other triangle cleared
-    if (!rows) {
-      for (int c = warp; c < sp::kNb; c += nw)
-        for (int r = lane; r < rest; r += 32) {
-          double2 v = zero;
-          if (c < nb && jb + r < k) {
-            if (r > c) v = L[jb + r + (long long)(jb + c) * n];
-            if (r == c) v = make_double2(1.0, 0.0);
-          }
-          T[r + c * ldt] = v;
-        }
-    } else {
-      for (int c = warp; c < rest; c += nw) {
-        const int r = lane;
-        double2 v = zero;
-        if (r < nb && jb + c < k && (r <= c)) v = L[jb + r + (long long)(jb + c) * n];
-        T[r + c * ldt] = v;
-      }
-    }
-    __syncthreads();
+    const int rest = kp - jb;  // from the block on, padded
     const int nt = rest / 8, nd = min(4, nt);
     if (!rows) {
       double2 *Xw = X + jb + 8 * warp * ldx;  // this warp's 8 columns, from row jb
@@ -458,37 +445,49 @@ __global__ void __launch_bounds__(kTrsmThreads)
       ZTile z[4];
 #pragma unroll
       for (int ti = 0; ti < 4; ti++)
-        if (ti < nd)
+        if (ti < nd) {
+          double2 a[8];
 #pragma unroll
-          for (int q = 0; q < 8; q++)
-            if (q <= 2 * ti + 1) z[ti].mma(T[8 * ti + lr + (4 * q + lk) * ldt], b[q]);
+          for (int q = 0; q <= 2 * ti + 1; q++) a[q] = at(jb + 8 * ti + lr, jb + 4 * q + lk);
+#pragma unroll
+          for (int q = 0; q <= 2 * ti + 1; q++) {
+            const int r = 8 * ti + lr, c = 4 * q + lk;  // strictly lower, unit diagonal
+            z[ti].mma(c < r ? a[q] : c == r ? one : zero, b[q]);
+          }
+        }
       __syncwarp();
 #pragma unroll
       for (int ti = 0; ti < 4; ti++)
         if (ti < nd)
 #pragma unroll
           for (int x = 0; x < 2; x++)
-            Xw[8 * ti + lr + (2 * lk + x) * ldx] = make_double2(z[ti].r[x], z[ti].i[x]);
+            if (jb + 8 * ti + lr < k)
+              Xw[8 * ti + lr + (2 * lk + x) * ldx] = make_double2(z[ti].r[x], z[ti].i[x]);
       __syncwarp();
 #pragma unroll
       for (int q = 0; q < 8; q++) b[q] = 4 * q < rest ? Xw[4 * q + lk + lr * ldx] : zero;
       for (int ti = 4; ti < nt; ti += 2) {
         ZTile y[2];
-        const bool two = ti + 1 < nt;
+        double2 a[2][8];
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int q = 0; q < 8; q++) a[h][q] = at(jb + 8 * (ti + h) + lr, jb + 4 * q + lk);
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-          y[0].mma(T[8 * ti + lr + (4 * q + lk) * ldt], b[q]);
-          if (two) y[1].mma(T[8 * ti + 8 + lr + (4 * q + lk) * ldt], b[q]);
+          y[0].mma(a[0][q], b[q]);
+          y[1].mma(a[1][q], b[q]);
         }
 #pragma unroll
         for (int h = 0; h < 2; h++)
-          if (h == 0 || two)
+          if (jb + 8 * (ti + h) + lr < k)
 #pragma unroll
             for (int x = 0; x < 2; x++) {
               double2 *o = Xw + 8 * (ti + h) + lr + (2 * lk + x) * ldx;
               *o = make_double2(o->x - y[h].r[x], o->y - y[h].i[x]);
             }
       }
+      __syncwarp();
     } else {
       double2 *Xw = X + 8 * warp + jb * ldx;  // this warp's 8 rows, from column jb
       double2 a[8];
@@ -497,45 +496,55 @@ __global__ void __launch_bounds__(kTrsmThreads)
       ZTile z[4];
 #pragma unroll
       for (int tj = 0; tj < 4; tj++)
-        if (tj < nd)
+        if (tj < nd) {
+          double2 b[8];
 #pragma unroll
-          for (int q = 0; q < 8; q++)
-            if (q <= 2 * tj + 1) z[tj].mma(a[q], T[4 * q + lk + (8 * tj + lr) * ldt]);
+          for (int q = 0; q <= 2 * tj + 1; q++) b[q] = at(jb + 4 * q + lk, jb + 8 * tj + lr);
+#pragma unroll
+          for (int q = 0; q <= 2 * tj + 1; q++)  // upper with the diagonal
+            z[tj].mma(a[q], 4 * q + lk <= 8 * tj + lr ? b[q] : zero);
+        }
       __syncwarp();
 #pragma unroll
       for (int tj = 0; tj < 4; tj++)
         if (tj < nd)
 #pragma unroll
           for (int x = 0; x < 2; x++)
-            Xw[lr + (8 * tj + 2 * lk + x) * ldx] = make_double2(z[tj].r[x], z[tj].i[x]);
+            if (jb + 8 * tj + 2 * lk + x < k)
+              Xw[lr + (8 * tj + 2 * lk + x) * ldx] = make_double2(z[tj].r[x], z[tj].i[x]);
       __syncwarp();
 #pragma unroll
       for (int q = 0; q < 8; q++) a[q] = 4 * q < rest ? Xw[lr + (4 * q + lk) * ldx] : zero;
       for (int tj = 4; tj < nt; tj += 2) {
         ZTile y[2];
-        const bool two = tj + 1 < nt;
+        double2 b[2][8];
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int q = 0; q < 8; q++) b[h][q] = at(jb + 4 * q + lk, jb + 8 * (tj + h) + lr);
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-          y[0].mma(a[q], T[4 * q + lk + (8 * tj + lr) * ldt]);
-          if (two) y[1].mma(a[q], T[4 * q + lk + (8 * tj + 8 + lr) * ldt]);
+          y[0].mma(a[q], b[0][q]);
+          y[1].mma(a[q], b[1][q]);
         }
 #pragma unroll
         for (int h = 0; h < 2; h++)
-          if (h == 0 || two)
 #pragma unroll
-            for (int x = 0; x < 2; x++) {
+          for (int x = 0; x < 2; x++)
+            if (jb + 8 * (tj + h) + 2 * lk + x < k) {
               double2 *o = Xw + lr + (8 * (tj + h) + 2 * lk + x) * ldx;
               *o = make_double2(o->x - y[h].r[x], o->y - y[h].i[x]);
             }
       }
+      __syncwarp();
     }
   }
-  __syncthreads();
   if (!rows) {
     double2 *U12 = L + (long long)n * k;
-    for (int c = warp; c < ns; c += nw)
+    for (int c = 8 * warp; c < min(8 * warp + 8, ns); c++)
       for (int r = lane; r < k; r += 32) U12[r + (long long)(s0 + c) * k] = X[r + c * ldx];
   } else {
+    __syncthreads();
     for (int c = warp; c < k; c += nw)
       if (lane < ns) L[k + s0 + lane + (long long)c * n] = X[lane + c * ldx];
   }
@@ -548,11 +557,13 @@ __global__ void __launch_bounds__(kTrsmThreads)
 // columns in registers (RPT rows a thread, chosen so that W RPT stays at 16),
 // each applied to the panel's columns to its right; then the diagonal block's
 // triangles are inverted in place.
-template <int W, int RPT>
-__global__ void __launch_bounds__(kPanelThreads)
+// SM: the panel stays in shared memory between its sub-panels (up to kSmRows rows).
+template <int W, int RPT, int T, bool SM>
+__global__ void __launch_bounds__(T)
     k_sp_panel(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
                double2 *__restrict__ work, int jb, int *__restrict__ swap, int *__restrict__ info) {
-  constexpr int T = kPanelThreads, kRight = sp::kNb - W;
+  constexpr int kRight = sp::kNb - W;
+  extern __shared__ double2 panel[];  // SM: [32][kSmLd]
   __shared__ PanelShared<W, T / 32> ps;
   __shared__ double2 Ls[W][W], Us[W][kRight > 0 ? kRight : 1];
   __shared__ int sdst[2 * W], ssrc[2 * W];
@@ -562,12 +573,21 @@ __global__ void __launch_bounds__(kPanelThreads)
   const SpFront f = fr[t];
   const int k = f.k;
   if (jb >= k) return;
-  const long long n = (long long)f.k + f.m;
+  const long long nf = (long long)f.k + f.m;
   const int nb = min(sp::kNb, k - jb), tid = threadIdx.x;
-  double2 *F = work + f.work0;
+  double2 *const G = work + f.work0 + jb * (nf + 1);  // the panel: rows and columns from jb
+  double2 *const F = SM ? panel : G;
+  const long long n = SM ? kSmLd : nf;
+  if (SM) {
+    for (int c = tid >> 5; c < nb; c += T / 32)
+      for (int r = tid & 31; r < k - jb; r += 32) cp16(F + r + c * n, G + r + c * nf, true);
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
+  }
   bool zero = false;
   for (int s0 = 0; s0 < nb; s0 += W) {
-    const int w = min(W, nb - s0), cb = jb + s0, nrow = k - cb;
+    const int w = min(W, nb - s0), cb = s0, nrow = k - jb - cb;  // cb: within the panel
     double2 a[RPT][W];
 #pragma unroll
     for (int q = 0; q < RPT; q++) {
@@ -589,7 +609,7 @@ __global__ void __launch_bounds__(kPanelThreads)
 #pragma unroll
       for (int c = 0; c < W; c++) Ls[tid][c] = a[0][c];
     __syncthreads();  // ps.swap complete
-    if (tid < w) swap[f.own0 + cb + tid] = cb + ps.swap[tid];
+    if (tid < w) swap[f.own0 + jb + cb + tid] = jb + cb + ps.swap[tid];
     if (tid < 2 * w) {
       const int d = tid < w ? tid : ps.swap[tid - w];
       sdst[tid] = d;
@@ -598,13 +618,22 @@ __global__ void __launch_bounds__(kPanelThreads)
     __syncthreads();
     // the interchanges on the panel's other columns
     {
-      const int i = tid % (2 * w), cc = tid / (2 * w);
-      const bool on = cc < nb - w;
-      const long long col = (cc < s0 ? jb + cc : cb + w + (cc - s0)) * n + cb;
-      double2 v = make_double2(0.0, 0.0);
-      if (on) v = F[col + ssrc[i]];
+      // 2 w rows of at most 32 - w columns: up to kPass rounds of T entries
+      constexpr int kPass = (2 * W * (sp::kNb - W) + T - 1) / T;
+      const int i = tid % (2 * w), per = T / (2 * w);
+      double2 v[kPass];
+#pragma unroll
+      for (int u = 0; u < kPass; u++) {
+        const int cc = tid / (2 * w) + u * per;
+        v[u] = cc < nb - w && tid < per * 2 * w ? F[(cc < s0 ? cc : cc + w) * n + cb + ssrc[i]]
+                                                : make_double2(0.0, 0.0);
+      }
       __syncthreads();
-      if (on) F[col + sdst[i]] = v;
+#pragma unroll
+      for (int u = 0; u < kPass; u++) {
+        const int cc = tid / (2 * w) + u * per;
+        if (cc < nb - w && tid < per * 2 * w) F[(cc < s0 ? cc : cc + w) * n + cb + sdst[i]] = v[u];
+      }
     }
     const int ncr = nb - s0 - w;
     if (ncr <= 0) break;
@@ -646,7 +675,7 @@ __global__ void __launch_bounds__(kPanelThreads)
   __syncthreads();
   for (int e = tid; e < sp::kNb * sp::kNb; e += T) {
     const int r = e % sp::kNb, c = e / sp::kNb;
-    if (r < nb && c < nb) D[c][r] = F[jb + r + (jb + c) * n];
+    if (r < nb && c < nb) D[c][r] = F[r + c * n];
   }
   __syncthreads();
   const int job = tid / (T / 2);
@@ -654,7 +683,12 @@ __global__ void __launch_bounds__(kPanelThreads)
                   dinv[job]);
   for (int e = tid; e < sp::kNb * sp::kNb; e += T) {
     const int r = e % sp::kNb, c = e / sp::kNb;
-    if (r < nb && c < nb) F[jb + r + (jb + c) * n] = D[c][r];
+    if (r < nb && c < nb) F[r + c * n] = D[c][r];
+  }
+  if (SM) {
+    __syncthreads();
+    for (int c = tid >> 5; c < nb; c += T / 32)
+      for (int r = tid & 31; r < k - jb; r += 32) G[r + c * nf] = F[r + c * n];
   }
 }
 
@@ -712,7 +746,7 @@ __global__ void __launch_bounds__(kPanelThreads)
     const double2 d = u[j];
     const bool z = !pivot_ok(d);
     zero |= z;
-    const double2 inv = z ? make_double2(0.0, 0.0) : cdiv(make_double2(1.0, 0.0), d);
+    const double2 inv = crecip(d);
     for (int r = jb + j + 1 + tid; r < k; r += T) {
       const double2 l = cmul(col[r], inv);
       col[r] = l;
@@ -864,17 +898,21 @@ __global__ void __launch_bounds__(kGemmThreads)
 // ---------------------------------------------------------------------------
 // products
 // ---------------------------------------------------------------------------
-// 64 x 64 tiles of C -= A B, four warps of 32 x 32 (4 x 4 tensor-core tiles of
-// complex 8 x 8), A and B staged by cp.async in double-buffered chunks of 8;
+// 32 x 32 tiles of C -= A B (t2 of them per front at most), four warps of 16 x 16 (2 x 2
+// tensor-core tiles of complex 8 x 8; at five CTAs an SM as fast as 64 x 64 tiles of
+// 4 x 4 where those are full, and 10 to 40 % faster where the fronts end in part
+// tiles: 15.3 against 19.0 ms over a factorisation of 331 GFLOP), A and B staged by cp.async in double-buffered chunks of 8;
 // 8 x 8 tiles past the edge are skipped.  jb < 0: the update F22 -= L21 U12 from
 // the factor store, K = k.  jb >= 0: the trailing update after panel jb of a
 // larger front, K = its columns, on rows and columns beyond the panel except
 // F22, in place in the work buffer.
-__global__ void __launch_bounds__(kGemmThreads, 3)
+__global__ void __launch_bounds__(kGemmThreads, 5)
     k_sp_gemm(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
-              double2 *__restrict__ work, const double2 *__restrict__ fac, int jb) {
+              double2 *__restrict__ work, const double2 *__restrict__ fac, int jb, int t2) {
+  constexpr int NT = kGt / 16;
   extern __shared__ double2 sh[];
-  const SpFront f = fr[fronts[blockIdx.x]];
+  const SpFront f = fr[fronts[blockIdx.x / t2]];
+  const int tile = blockIdx.x % t2;
   const int k = f.k, m = f.m, n = k + m;
   const double2 *A, *B;
   double2 *C;
@@ -899,21 +937,21 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     C = work + f.work0 + (long long)c1 * (n + 1);
     corner = k - c1;
   }
-  const int tiles = (M + kTile - 1) / kTile;
-  if (K == 0 || (int)blockIdx.y >= tiles * tiles) return;
-  const int m0 = ((int)blockIdx.y % tiles) * kTile, n0 = ((int)blockIdx.y / tiles) * kTile;
+  const int tiles = (M + kGt - 1) / kGt;
+  if (K == 0 || tile >= tiles * tiles) return;
+  const int m0 = (tile % tiles) * kGt, n0 = (tile / tiles) * kGt;
   if (m0 >= corner && n0 >= corner && jb >= 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lk = lane & 3;
-  const int wm = 32 * (warp & 1), wn = 32 * (warp >> 1);
-  const int mt = min(4, max(0, (M - m0 - wm + 7) / 8)), nt = min(4, max(0, (M - n0 - wn + 7) / 8));
+  const int wm = kGt / 2 * (warp & 1), wn = kGt / 2 * (warp >> 1);
+  const int mt = min(NT, max(0, (M - m0 - wm + 7) / 8)), nt = min(NT, max(0, (M - n0 - wn + 7) / 8));
   auto stage = [&](int ch) {
     double2 *As = sh + (ch & 1) * kGemmStage, *Bs = As + kKc * kGemmLda;
     const int k0 = ch * kKc;
 #pragma unroll
-    for (int q = 0; q < kKc * kTile / kGemmThreads; q++) {
+    for (int q = 0; q < kKc * kGt / kGemmThreads; q++) {
       const int e = tid + q * kGemmThreads;
       {
-        const int r = e % kTile, c = e / kTile;
+        const int r = e % kGt, c = e / kGt;
         const bool ok = m0 + r < M && k0 + c < K;
         cp16(As + r + c * kGemmLda, ok ? A + m0 + r + (long long)(k0 + c) * lda : A, ok);
       }
@@ -925,7 +963,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     }
     cp_commit();
   };
-  ZTile z[4][4];
+  ZTile z[NT][NT];
   const int nch = (K + kKc - 1) / kKc;
   stage(0);
   for (int ch = 0; ch < nch; ch++) {
@@ -939,15 +977,15 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     const double2 *As = sh + (ch & 1) * kGemmStage, *Bs = As + kKc * kGemmLda;
 #pragma unroll
     for (int kk = 0; kk < kKc; kk += 4) {
-      double2 b[4];
+      double2 b[NT];
 #pragma unroll
-      for (int tj = 0; tj < 4; tj++) b[tj] = Bs[kk + lk + (wn + 8 * tj + lr) * kGemmLdb];
+      for (int tj = 0; tj < NT; tj++) b[tj] = Bs[kk + lk + (wn + 8 * tj + lr) * kGemmLdb];
 #pragma unroll
-      for (int ti = 0; ti < 4; ti++) {
+      for (int ti = 0; ti < NT; ti++) {
         if (ti < mt) {
           const double2 a = As[wm + 8 * ti + lr + (kk + lk) * kGemmLda];
 #pragma unroll
-          for (int tj = 0; tj < 4; tj++)
+          for (int tj = 0; tj < NT; tj++)
             if (tj < nt) z[ti][tj].mma(a, b[tj]);
         }
       }
@@ -955,9 +993,9 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     __syncthreads();
   }
 #pragma unroll
-  for (int ti = 0; ti < 4; ti++)
+  for (int ti = 0; ti < NT; ti++)
 #pragma unroll
-    for (int tj = 0; tj < 4; tj++)
+    for (int tj = 0; tj < NT; tj++)
 #pragma unroll
       for (int x = 0; x < 2; x++) {
         const int r = m0 + wm + 8 * ti + lr, c = n0 + wn + 8 * tj + 2 * lk + x;
@@ -990,10 +1028,10 @@ __global__ void k_sp_store(const int *__restrict__ fronts, const SpFront *__rest
 size_t lu_smem(int k) { return sizeof(double2) * (size_t)k * (k | 1); }
 size_t trsm_smem(int kmax) {
   const size_t kp = (kmax + 7) & ~7;
-  return sizeof(double2) * std::max((kp + 5) * kStrip + (kp + 2) * sp::kNb,
-                                    (kStrip + 2) * kp + (sp::kNb + 4) * kp);
+  return sizeof(double2) * (kp + 5) * (kStrip + 2);
 }
 constexpr size_t kApplySmem = sizeof(double2) * (kTile + sp::kNb) * (sp::kNb + 4);
+constexpr size_t kPanelSmem = sizeof(double2) * sp::kNb * kSmLd;
 constexpr size_t kGemmSmem = sizeof(double2) * 2 * kGemmStage;
 
 }  // namespace
@@ -1006,11 +1044,15 @@ cudaError_t sparse_factor_attributes() {
   if ((e = cudaFuncSetAttribute(k_sp_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)trsm_smem(sp::kSmallK))))
     return e;
+  if ((e = cudaFuncSetAttribute(k_sp_panel<8, 1, kSmThreads, true>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem)) ||
+      (e = cudaFuncSetAttribute(k_sp_panel<8, 2, kSmThreads, true>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem)))
+    return e;
   if ((e = cudaFuncSetAttribute(k_sp_panel_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kApplySmem)))
     return e;
-  return cudaFuncSetAttribute(k_sp_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)kGemmSmem);
+  return cudaSuccess;
 }
 
 cudaError_t sparse_factor_level(SparseLU *s, int l, const double2 *csr, double2 *W,
@@ -1041,28 +1083,41 @@ cudaError_t sparse_factor_level(SparseLU *s, int l, const double2 *csr, double2 
     const int cap = env ? std::atoi(env) : 8;
     for (int jb = 0; jb < kmax; jb += sp::kNb) {
       const int rows = kmax - jb;
-      if (rows <= kPanelThreads && cap >= 8)
-        k_sp_panel<8, 1><<<nbig, kPanelThreads, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
-      else if (rows <= 2 * kPanelThreads && cap >= 8)
-        k_sp_panel<8, 2><<<nbig, kPanelThreads, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
-      else if (rows <= 4 * kPanelThreads && cap >= 4)
-        k_sp_panel<4, 4><<<nbig, kPanelThreads, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
-      else if (rows <= 8 * kPanelThreads && cap >= 2)
-        k_sp_panel<2, 8><<<nbig, kPanelThreads, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
+      constexpr int PT = kPanelThreads, ST = kSmThreads;
+      if (rows <= ST && cap >= 8)
+        k_sp_panel<8, 1, ST, true>
+            <<<nbig, ST, kPanelSmem, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
+      else if (rows <= kSmRows && cap >= 8)
+        k_sp_panel<8, 2, ST, true>
+            <<<nbig, ST, kPanelSmem, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
+      else if (rows <= PT && cap >= 8)
+        k_sp_panel<8, 1, PT, false>
+            <<<nbig, PT, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
+      else if (rows <= 2 * PT && cap >= 8)
+        k_sp_panel<8, 2, PT, false>
+            <<<nbig, PT, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
+      else if (rows <= 4 * PT && cap >= 4)
+        k_sp_panel<4, 4, PT, false>
+            <<<nbig, PT, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
+      else if (rows <= 8 * PT && cap >= 2)
+        k_sp_panel<2, 8, PT, false>
+            <<<nbig, PT, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
       else
         k_sp_panel_any<<<nbig, kPanelThreads, 0, st>>>(big, s->d_fr, W, jb, s->d_swap, s->d_info);
       const int right = nmax - jb;  // >= columns beyond the panel of any front
       k_sp_panel_apply<<<dim3(nbig, tiles(right) + tiles(jb) + tiles(mmax) + 1), kGemmThreads,
                          kApplySmem, st>>>(big, s->d_fr, W, jb, s->d_swap);
-      k_sp_gemm<<<dim3(nbig, tiles(right) * tiles(right)), kGemmThreads, kGemmSmem, st>>>(
-          big, s->d_fr, W, s->d_fac, jb);
+      const int tr = (right + kGt - 1) / kGt;
+      k_sp_gemm<<<(unsigned)(nbig * tr * tr), kGemmThreads, kGemmSmem, st>>>(
+          big, s->d_fr, W, s->d_fac, jb, tr * tr);
     }
     const unsigned ysb = (unsigned)std::max(1, std::min(256, 8 * nsm / nbig));
     k_sp_store<<<dim3(nbig, ysb), 256, 0, st>>>(big, s->d_fr, W, s->d_fac, s->d_swap, s->d_perm);
   }
   if (s->lev_mmax[l] > 0) {
-    const int tm = tiles(s->lev_mmax[l]);
-    k_sp_gemm<<<dim3(nfl, tm * tm), kGemmThreads, kGemmSmem, st>>>(dfr, s->d_fr, W, s->d_fac, -1);
+    const int tm = (s->lev_mmax[l] + kGt - 1) / kGt;
+    k_sp_gemm<<<(unsigned)((long long)nfl * tm * tm), kGemmThreads, kGemmSmem, st>>>(
+        dfr, s->d_fr, W, s->d_fac, -1, tm * tm);
   }
   return cudaGetLastError();
 }
