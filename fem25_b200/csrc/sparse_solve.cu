@@ -942,7 +942,8 @@ __global__ void __launch_bounds__(kTriThreads) k_sp_tri_any(SolveArgs a, int fwd
 // backward y -= rect x_b.
 template <int NT>
 __global__ void __launch_bounds__(256) k_sp_rect(SolveArgs a, int fwd) {
-  constexpr int ld = 8 * NT + 2;
+  // longer chunks where the columns are few: 40 KB of shared memory for any NT
+  constexpr int ld = 8 * NT + 2, kChunk = 256 / NT;
   __shared__ double2 Y[kChunk * ld];
   const SpFront f = a.fr[a.fronts[blockIdx.x]];
   const SpStep st(a, f, fwd);
