@@ -13,6 +13,7 @@ namespace sp {
 constexpr int kLeafElems = 2;  // elements per leaf of the dissection
 constexpr int kNb = 32;        // columns of a panel and of an inverted diagonal block
 constexpr int kSmallK = 96;    // fronts with at most this many own DOFs: F11 in shared memory
+constexpr int kStreams = 3;    // groups of a level's fronts factored side by side
 }  // namespace sp
 
 struct SpFront {
@@ -54,6 +55,11 @@ struct SparseLU {
   int *d_swap = nullptr;               // [NDOF] interchanges of the panels being factored
   double2 *d_work[2] = {nullptr, nullptr};
   int *d_info = nullptr;               // first zero pivot (front + 1), 0 = none
+  // per group of fronts: its stream, a side stream for the updates that the next
+  // panel does not wait for, and the events between them and the caller's stream
+  cudaStream_t st[sp::kStreams] = {}, side[sp::kStreams] = {};
+  cudaEvent_t done[sp::kStreams] = {}, applied[sp::kStreams] = {}, updated[sp::kStreams] = {};
+  cudaEvent_t ready = nullptr;
 };
 
 // Numeric factorisation of one level's fronts (sparse_factor.cu): W holds the

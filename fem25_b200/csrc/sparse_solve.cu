@@ -979,6 +979,13 @@ void free_sparse(Ctx *c) {
                   s->d_info};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  for (int g = 0; g < sp::kStreams; g++) {
+    for (cudaStream_t q : {s->st[g], s->side[g]})
+      if (q) cudaStreamDestroy(q);
+    for (cudaEvent_t q : {s->done[g], s->applied[g], s->updated[g]})
+      if (q) cudaEventDestroy(q);
+  }
+  if (s->ready) cudaEventDestroy(s->ready);
   delete s;
   c->sparse = nullptr;
 }
@@ -1029,6 +1036,19 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
   SPCK(sparse_solve_attributes<1>(), "kernel attributes");
   SPCK(sparse_solve_attributes<2>(), "kernel attributes");
   SPCK(sparse_solve_attributes<4>(), "kernel attributes");
+  if (!s->ready) {
+    // the groups' own streams go before their side streams: a panel must not queue
+    // behind the update beside it
+    int least = 0, greatest = 0;
+    SPCK(cudaDeviceGetStreamPriorityRange(&least, &greatest), "streams");
+    for (int g = 0; g < sp::kStreams; g++) {
+      SPCK(cudaStreamCreateWithPriority(&s->st[g], cudaStreamNonBlocking, greatest), "streams");
+      SPCK(cudaStreamCreateWithPriority(&s->side[g], cudaStreamNonBlocking, least), "streams");
+      for (cudaEvent_t *q : {&s->done[g], &s->applied[g], &s->updated[g]})
+        SPCK(cudaEventCreateWithFlags(q, cudaEventDisableTiming), "events");
+    }
+    SPCK(cudaEventCreateWithFlags(&s->ready, cudaEventDisableTiming), "events");
+  }
   if (!s->d_fac) {
     SPCK(cudaMalloc(&s->d_fac, sizeof(double2) * std::max(s->fac_elems, 1LL)), "factor store");
     SPCK(cudaMalloc(&s->d_perm, sizeof(int) * std::max(c->ndof, 1)), "pivots");
