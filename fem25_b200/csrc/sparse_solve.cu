@@ -1049,14 +1049,16 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
     }
     SPCK(cudaEventCreateWithFlags(&s->ready, cudaEventDisableTiming), "events");
   }
-  if (!s->d_fac) {
-    SPCK(cudaMalloc(&s->d_fac, sizeof(double2) * std::max(s->fac_elems, 1LL)), "factor store");
-    SPCK(cudaMalloc(&s->d_perm, sizeof(int) * std::max(c->ndof, 1)), "pivots");
-    SPCK(cudaMalloc(&s->d_swap, sizeof(int) * std::max(c->ndof, 1)), "pivots");
-    SPCK(cudaMalloc(&s->d_work[0], sizeof(double2) * std::max(s->max_work, 1LL)), "work");
-    SPCK(cudaMalloc(&s->d_work[1], sizeof(double2) * std::max(s->max_work, 1LL)), "work");
-    SPCK(cudaMalloc(&s->d_info, sizeof(int)), "status");
-  }
+  // each by itself: a call after one that ran out of memory makes what is missing
+  auto keep = [](auto **p, size_t n) {
+    return *p ? cudaSuccess : cudaMalloc(p, sizeof(**p) * std::max(n, (size_t)1));
+  };
+  SPCK(keep(&s->d_fac, (size_t)s->fac_elems), "factor store");
+  SPCK(keep(&s->d_perm, (size_t)c->ndof), "pivots");
+  SPCK(keep(&s->d_swap, (size_t)c->ndof), "pivots");
+  SPCK(keep(&s->d_work[0], (size_t)s->max_work), "work");
+  SPCK(keep(&s->d_work[1], (size_t)s->max_work), "work");
+  SPCK(keep(&s->d_info, 1), "status");
   SPCK(cudaMemsetAsync(s->d_info, 0, sizeof(int), st), "status");
   const double2 *csr = reinterpret_cast<const double2 *>(csr128);
   int nsm = 0;
