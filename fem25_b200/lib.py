@@ -310,7 +310,7 @@ class Context:
             pass
 
     def tuning(self):
-        """Autotuner choices: {"stream_variant": v, "grad_tile": t} (-1 = not tuned)."""
+        """Kernel variants picked so far: {"stream_variant": v, "grad_tile": t} (-1 = none yet)."""
         v, t = C.c_int(), C.c_int()
         lib().fem25_tuning(self.h, C.byref(v), C.byref(t))
         return {"stream_variant": v.value, "grad_tile": t.value}
