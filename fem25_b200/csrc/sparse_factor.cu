@@ -1,7 +1,7 @@
 // Numeric factorisation of the sparse direct solve's fronts, one level of the
 // dissection tree at a time (the tree, the fronts and their storage are
 // described in sparse_solve.cu).  Per level:
-//   k_sp_pull       every front = the update blocks of its two children
+//   k_sp_pull       F11, F12, F21 = the update blocks of its two children
 //   k_sp_entries    + the CSR entries whose first eliminated DOF it owns
 //   F11 = P L11 U11, partial pivoting among the fully summed rows:
 //     k <= 96       k_sp_lu (F11 in shared memory), then k_sp_trsm for
@@ -9,7 +9,7 @@
 //     larger        panels of 32 columns: k_sp_panel, k_sp_panel_apply (row
 //                   interchanges, the panel's rows of U, its part of L21),
 //                   k_sp_gemm (trailing update of everything but F22)
-//   k_sp_gemm       F22 -= L21 U12, once, over all k
+//   k_sp_gemm       F22 = the children's update blocks - L21 U12, once, over all k
 // What bounds it: FP64 operations, 8/3 k^3 + 8 k^2 m + 8 k m^2 a front, most of
 // them in products.  The products run on the FP64 tensor cores (mma m8n8k4;
 // measured 36.9 TFLOP/s against 36.6 for DFMA, but an operand read from shared
@@ -40,30 +40,44 @@ constexpr int kGemmStage = kKc * kGemmLda + kGt * kGemmLdb;  // double2 per stag
 // Front entry (i, j) = its two children's update entries at (map[i], map[j]),
 // where map is the position in the child's boundary or -1: the child's update
 // block starts at row and column k of its front.  Every entry is written once,
-// so nothing is cleared first and no child is added by read-modify-write.
+// so nothing is cleared first and no child is added by read-modify-write.  F22,
+// most of a front, is left to k_sp_gemm, which takes the children's entries in as it
+// writes it (written here and read back there it cost 36.0 ms instead of 34.0 over a
+// factorisation of 331 GFLOP and a solve).
+struct Children {
+  const int *map[2];
+  const double2 *base[2] = {nullptr, nullptr};
+  long long ld[2] = {0, 0};
+  __device__ __forceinline__ Children(const SpFront &f, const SpFront *__restrict__ fr,
+                                      const int *__restrict__ pull,
+                                      const double2 *__restrict__ wchild) {
+    map[0] = pull + f.map0;
+    map[1] = map[0] + f.k + f.m;
+    for (int s = 0; s < 2; s++)
+      if (f.child[s] >= 0) {
+        const SpFront g = fr[f.child[s]];
+        ld[s] = (long long)g.k + g.m;
+        base[s] = wchild + g.work0 + g.k * (ld[s] + 1);
+      }
+  }
+};
+
 __global__ void k_sp_pull(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
                           const int *__restrict__ pull, const double2 *__restrict__ wchild,
                           double2 *__restrict__ work) {
   const SpFront f = fr[fronts[blockIdx.x]];
   const int n = f.k + f.m;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int *map[2] = {pull + f.map0, pull + f.map0 + n};
-  const double2 *base[2] = {nullptr, nullptr};
-  long long ld[2] = {0, 0};
-  for (int s = 0; s < 2; s++)
-    if (f.child[s] >= 0) {
-      const SpFront g = fr[f.child[s]];
-      ld[s] = (long long)g.k + g.m;
-      base[s] = wchild + g.work0 + g.k * (ld[s] + 1);
-    }
+  const Children ch(f, fr, pull, wchild);
   for (int j = blockIdx.y * nw + (threadIdx.x >> 5); j < n; j += gridDim.y * nw) {
-    const int j0 = base[0] ? map[0][j] : -1, j1 = base[1] ? map[1][j] : -1;
+    const int j0 = ch.base[0] ? ch.map[0][j] : -1, j1 = ch.base[1] ? ch.map[1][j] : -1;
     double2 *dst = work + f.work0 + (long long)j * n;
-    const double2 *c0 = base[0] + j0 * ld[0], *c1 = base[1] + j1 * ld[1];
+    const double2 *c0 = ch.base[0] + j0 * ch.ld[0], *c1 = ch.base[1] + j1 * ch.ld[1];
+    const int rows = j < f.k ? n : f.k;
 #pragma unroll 2
-    for (int i = lane; i < n; i += 32) {
+    for (int i = lane; i < rows; i += 32) {
       double2 v = make_double2(0.0, 0.0);
-      const int i0 = j0 >= 0 ? map[0][i] : -1, i1 = j1 >= 0 ? map[1][i] : -1;
+      const int i0 = j0 >= 0 ? ch.map[0][i] : -1, i1 = j1 >= 0 ? ch.map[1][i] : -1;
       if (i0 >= 0) v = c0[i0];
       if (i1 >= 0) {
         const double2 w = c1[i1];
@@ -902,13 +916,15 @@ __global__ void __launch_bounds__(kGemmThreads)
 // tensor-core tiles of complex 8 x 8; at five CTAs an SM as fast as 64 x 64 tiles of
 // 4 x 4 where those are full, and 10 to 40 % faster where the fronts end in part
 // tiles: 15.3 against 19.0 ms over a factorisation of 331 GFLOP), A and B staged by cp.async in double-buffered chunks of 8;
-// 8 x 8 tiles past the edge are skipped.  jb < 0: the update F22 -= L21 U12 from
-// the factor store, K = k.  jb >= 0: the trailing update after panel jb of a
-// larger front, K = its columns, on rows and columns beyond the panel except
-// F22, in place in the work buffer.
+// 8 x 8 tiles past the edge are skipped.  SCHUR: F22 = the children's updates -
+// L21 U12 from the factor store, K = k (jb unused).  Otherwise the trailing update
+// after panel jb of a larger front, K = its columns, on rows and columns beyond the
+// panel except F22, in place in the work buffer.
+template <bool SCHUR>
 __global__ void __launch_bounds__(kGemmThreads, 5)
     k_sp_gemm(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
-              double2 *__restrict__ work, const double2 *__restrict__ fac, int jb, int t2, int c0, int cn) {
+              double2 *__restrict__ work, const double2 *__restrict__ fac, int jb, int t2, int c0,
+              int cn, const int *__restrict__ pull, const double2 *__restrict__ wchild) {
   constexpr int NT = kGt / 16;
   extern __shared__ double2 sh[];
   const SpFront f = fr[fronts[blockIdx.x / t2]];
@@ -916,8 +932,9 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
   const int k = f.k, m = f.m, n = k + m;
   const double2 *A, *B;
   double2 *C;
-  int M, K, lda, ldb, corner;  // corner: C(r, c) with r, c >= corner is left alone
-  if (jb < 0) {
+  int M, K, lda, ldb;
+  [[maybe_unused]] int corner = 0;  // C(r, c) with r, c >= corner is left alone
+  if (SCHUR) {
     M = m;
     K = k;
     A = fac + f.fac0 + k;
@@ -925,7 +942,6 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
     B = fac + f.fac0 + (long long)n * k;
     ldb = k;
     C = work + f.work0 + (long long)k * (n + 1);
-    corner = M;
   } else {
     if (jb >= k) return;
     K = min(sp::kNb, k - jb);
@@ -939,9 +955,9 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
   }
   const int tiles = (M + kGt - 1) / kGt;
   const int tc = tile / tiles;
-  if (K == 0 || tc >= cn || c0 + tc >= tiles) return;
+  if ((!SCHUR && K == 0) || tc >= cn || c0 + tc >= tiles) return;
   const int m0 = (tile - tc * tiles) * kGt, n0 = (c0 + tc) * kGt;
-  if (m0 >= corner && n0 >= corner && jb >= 0) return;
+  if (!SCHUR && m0 >= corner && n0 >= corner) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lk = lane & 3;
   const int wm = kGt / 2 * (warp & 1), wn = kGt / 2 * (warp >> 1);
   const int mt = min(NT, max(0, (M - m0 - wm + 7) / 8)), nt = min(NT, max(0, (M - n0 - wn + 7) / 8));
@@ -966,7 +982,7 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
   };
   ZTile z[NT][NT];
   const int nch = (K + kKc - 1) / kKc;
-  stage(0);
+  if (nch > 0) stage(0);
   for (int ch = 0; ch < nch; ch++) {
     if (ch + 1 < nch) {
       stage(ch + 1);
@@ -993,6 +1009,40 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
     }
     __syncthreads();
   }
+  if (SCHUR) {
+    const Children ch(f, fr, pull, wchild);
+    int row[2][NT], col[2][2 * NT];  // places in the children's boundaries
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+#pragma unroll
+      for (int ti = 0; ti < NT; ti++) {
+        const int r = m0 + wm + 8 * ti + lr;
+        row[s][ti] = ch.base[s] && r < M ? ch.map[s][k + r] : -1;
+      }
+#pragma unroll
+      for (int q = 0; q < 2 * NT; q++) {
+        const int c = n0 + wn + 8 * (q >> 1) + 2 * lk + (q & 1);
+        col[s][q] = ch.base[s] && c < M ? ch.map[s][k + c] : -1;
+      }
+    }
+#pragma unroll
+    for (int ti = 0; ti < NT; ti++)
+#pragma unroll
+      for (int q = 0; q < 2 * NT; q++) {
+        const int r = m0 + wm + 8 * ti + lr, c = n0 + wn + 8 * (q >> 1) + 2 * lk + (q & 1);
+        double2 v = make_double2(0.0, 0.0);
+        if (row[0][ti] >= 0 && col[0][q] >= 0) v = ch.base[0][row[0][ti] + col[0][q] * ch.ld[0]];
+        if (row[1][ti] >= 0 && col[1][q] >= 0) {
+          const double2 w = ch.base[1][row[1][ti] + col[1][q] * ch.ld[1]];
+          v.x += w.x;
+          v.y += w.y;
+        }
+        const ZTile &t = z[ti][q >> 1];
+        if (r < M && c < M)
+          C[r + (long long)c * n] = make_double2(v.x - t.r[q & 1], v.y - t.i[q & 1]);
+      }
+    return;
+  }
 #pragma unroll
   for (int ti = 0; ti < NT; ti++)
 #pragma unroll
@@ -1000,7 +1050,7 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
 #pragma unroll
       for (int x = 0; x < 2; x++) {
         const int r = m0 + wm + 8 * ti + lr, c = n0 + wn + 8 * tj + 2 * lk + x;
-        if (r < M && c < M && !(jb >= 0 && r >= corner && c >= corner)) {
+        if (r < M && c < M && !(r >= corner && c >= corner)) {
           double2 *o = C + r + (long long)c * n;
           *o = make_double2(o->x - z[ti][tj].r[x], o->y - z[ti][tj].i[x]);
         }
@@ -1058,7 +1108,7 @@ cudaError_t sparse_factor_attributes() {
 
 // nf of level l's fronts (with k <= kSmallK or larger) on group g's streams
 static cudaError_t factor_group(SparseLU *s, int l, const int *fronts, int nf, bool small,
-                                double2 *W, int nsm, int g) {
+                                double2 *W, const double2 *Wc, int nsm, int g) {
   if (nf <= 0) return cudaSuccess;
   const cudaStream_t st = s->st[g];
   cudaError_t e;
@@ -1107,14 +1157,15 @@ static cudaError_t factor_group(SparseLU *s, int l, const int *fronts, int nf, b
                          kApplySmem, st>>>(fronts, s->d_fr, W, jb, s->d_swap);
       const int tr = (right + kGt - 1) / kGt;
       // the next panel's columns on this stream, the others beside it
-      k_sp_gemm<<<(unsigned)(nf * tr), kGemmThreads, kGemmSmem, st>>>(fronts, s->d_fr, W, s->d_fac,
-                                                                    jb, tr, 0, 1);
+      k_sp_gemm<false><<<(unsigned)(nf * tr), kGemmThreads, kGemmSmem, st>>>(
+          fronts, s->d_fr, W, s->d_fac, jb, tr, 0, 1, nullptr, nullptr);
       if (tr > 1) {
         if ((e = cudaEventRecord(s->applied[g], st)) ||
             (e = cudaStreamWaitEvent(s->side[g], s->applied[g], 0)))
           return e;
-        k_sp_gemm<<<(unsigned)(nf * tr * (tr - 1)), kGemmThreads, kGemmSmem, s->side[g]>>>(
-            fronts, s->d_fr, W, s->d_fac, jb, tr * (tr - 1), 1, tr - 1);
+        k_sp_gemm<false>
+            <<<(unsigned)(nf * tr * (tr - 1)), kGemmThreads, kGemmSmem, s->side[g]>>>(
+                fronts, s->d_fr, W, s->d_fac, jb, tr * (tr - 1), 1, tr - 1, nullptr, nullptr);
         if ((e = cudaEventRecord(s->updated[g], s->side[g]))) return e;
         pending = true;
       }
@@ -1126,8 +1177,8 @@ static cudaError_t factor_group(SparseLU *s, int l, const int *fronts, int nf, b
   const int mmax = small ? s->lev_msmall[l] : s->lev_mmax[l];
   if (mmax > 0) {
     const int tm = (mmax + kGt - 1) / kGt;
-    k_sp_gemm<<<(unsigned)((long long)nf * tm * tm), kGemmThreads, kGemmSmem, st>>>(
-        fronts, s->d_fr, W, s->d_fac, -1, tm * tm, 0, tm);
+    k_sp_gemm<true><<<(unsigned)((long long)nf * tm * tm), kGemmThreads, kGemmSmem, st>>>(
+        fronts, s->d_fr, W, s->d_fac, -1, tm * tm, 0, tm, s->d_pull, Wc);
   }
   return cudaSuccess;
 }
@@ -1145,7 +1196,8 @@ cudaError_t sparse_factor_level(SparseLU *s, int l, const double2 *csr, double2 
         ne, s->d_ent_idx + s->lev_ent0[l], s->d_ent_loc + s->lev_ent0[l], csr, W);
   // The fronts in groups, each on a stream of its own: a group's pivot searches (one
   // CTA a front) run beside another's products, and within a group the next panel
-  // beside the update of the columns behind it.  38.7 ms on one stream, 37.4 in
+  // beside the update of the columns behind it.  Before F22's sums moved into the
+  // products (the line above k_sp_pull): 38.7 ms on one stream, 37.4 in
   // groups, 36.2 with the side streams, 35.7 with the groups' streams first in
   // priority (2 to 4 groups within 1 %, 8 slower).
   cudaError_t e;
@@ -1156,8 +1208,8 @@ cudaError_t sparse_factor_level(SparseLU *s, int l, const double2 *csr, double2 
     if ((e = cudaStreamWaitEvent(sg, s->ready, 0))) return e;
     const int a0 = (int)((long long)nsmall * g / groups), a1 = (int)((long long)nsmall * (g + 1) / groups);
     const int b0 = (int)((long long)nbig * g / groups), b1 = (int)((long long)nbig * (g + 1) / groups);
-    if ((e = factor_group(s, l, dfr + a0, a1 - a0, true, W, nsm, g)) ||
-        (e = factor_group(s, l, dfr + nsmall + b0, b1 - b0, false, W, nsm, g)) ||
+    if ((e = factor_group(s, l, dfr + a0, a1 - a0, true, W, Wc, nsm, g)) ||
+        (e = factor_group(s, l, dfr + nsmall + b0, b1 - b0, false, W, Wc, nsm, g)) ||
         (e = cudaEventRecord(s->done[g], sg)) || (e = cudaStreamWaitEvent(st, s->done[g], 0)))
       return e;
   }
