@@ -912,14 +912,15 @@ __global__ void __launch_bounds__(kGemmThreads)
 // ---------------------------------------------------------------------------
 // products
 // ---------------------------------------------------------------------------
-// 32 x 32 tiles of C -= A B, tile columns [c0, c0 + cn) (t2 tiles per front at most), four warps of 16 x 16 (2 x 2
-// tensor-core tiles of complex 8 x 8; at five CTAs an SM as fast as 64 x 64 tiles of
-// 4 x 4 where those are full, and 10 to 40 % faster where the fronts end in part
-// tiles: 15.3 against 19.0 ms over a factorisation of 331 GFLOP), A and B staged by cp.async in double-buffered chunks of 8;
-// 8 x 8 tiles past the edge are skipped.  SCHUR: F22 = the children's updates -
-// L21 U12 from the factor store, K = k (jb unused).  Otherwise the trailing update
-// after panel jb of a larger front, K = its columns, on rows and columns beyond the
-// panel except F22, in place in the work buffer.
+// 32 x 32 tiles of C -= A B, tile columns [c0, c0 + cn) (t2 tiles per front at
+// most), four warps of 16 x 16 (2 x 2 tensor-core tiles of complex 8 x 8; at five CTAs
+// an SM as fast as 64 x 64 tiles of 4 x 4 where those are full, and 10 to 40 % faster
+// where the fronts end in part tiles: 15.3 against 19.0 ms over a factorisation of
+// 331 GFLOP), A and B staged by cp.async in double-buffered chunks of 8; 8 x 8 tiles
+// past the edge are skipped.  SCHUR: F22 = the children's updates - L21 U12 from the
+// factor store, K = k (jb unused).  Otherwise the trailing update after panel jb of a
+// larger front, K = its columns, on rows and columns beyond the panel except F22, in
+// place in the work buffer.
 template <bool SCHUR>
 __global__ void __launch_bounds__(kGemmThreads, 5)
     k_sp_gemm(const int *__restrict__ fronts, const SpFront *__restrict__ fr,
