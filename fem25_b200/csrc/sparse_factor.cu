@@ -20,6 +20,7 @@
 #include <cstdlib>
 
 #include "sparse.cuh"
+#include "sparse_tiles.h"
 
 namespace fem25 {
 
@@ -30,7 +31,8 @@ constexpr int kSmThreads = 256, kSmRows = 390, kSmLd = kSmRows + 1;  // panel in
 constexpr int kLuThreads = 256;
 constexpr int kLuRows = 128;     // threads of k_sp_lu that hold a row of a sub-panel
 constexpr int kTrsmThreads = 128, kStrip = 32;
-constexpr int kGemmThreads = 128, kTile = 64, kGt = 32, kKc = 8;
+using sp::kGt;
+constexpr int kGemmThreads = 128, kTile = 64, kKc = 8;
 constexpr int kGemmLda = kGt + 2, kGemmLdb = kKc + 4;  // conflict-free fragment reads
 constexpr int kGemmStage = kKc * kGemmLda + kGt * kGemmLdb;  // double2 per stage
 
@@ -934,9 +936,9 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
   const double2 *A, *B;
   double2 *C;
   int M, K, lda, ldb;
-  [[maybe_unused]] int corner = 0;  // C(r, c) with r, c >= corner is left alone
+  int corner;  // C(r, c) with r, c >= corner is left alone
   if (SCHUR) {
-    M = m;
+    M = corner = m;
     K = k;
     A = fac + f.fac0 + k;
     lda = n;
@@ -954,11 +956,8 @@ __global__ void __launch_bounds__(kGemmThreads, 5)
     C = work + f.work0 + (long long)c1 * (n + 1);
     corner = k - c1;
   }
-  const int tiles = (M + kGt - 1) / kGt;
-  const int tc = tile / tiles;
-  if ((!SCHUR && K == 0) || tc >= cn || c0 + tc >= tiles) return;
-  const int m0 = (tile - tc * tiles) * kGt, n0 = (c0 + tc) * kGt;
-  if (!SCHUR && m0 >= corner && n0 >= corner) return;
+  int m0, n0;
+  if (!sp::gemm_tile(M, corner, tile, c0, cn, &m0, &n0)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lk = lane & 3;
   const int wm = kGt / 2 * (warp & 1), wn = kGt / 2 * (warp >> 1);
   const int mt = min(NT, max(0, (M - m0 - wm + 7) / 8)), nt = min(NT, max(0, (M - n0 - wn + 7) / 8));
@@ -1156,6 +1155,7 @@ static cudaError_t factor_group(SparseLU *s, int l, const int *fronts, int nf, b
       const int right = nmax - jb;  // >= columns beyond the panel of any front
       k_sp_panel_apply<<<dim3(nf, tiles(right) + tiles(jb) + tiles(mmax) + 1), kGemmThreads,
                          kApplySmem, st>>>(fronts, s->d_fr, W, jb, s->d_swap);
+      if (kmax <= jb + sp::kNb) break;  // the last panel: only F22 lies beyond it
       const int tr = (right + kGt - 1) / kGt;
       // the next panel's columns on this stream, the others beside it
       k_sp_gemm<false><<<(unsigned)(nf * tr), kGemmThreads, kGemmSmem, st>>>(
