@@ -107,27 +107,45 @@ __global__ void k_sp_entries(long long n, const int *__restrict__ idx,
 // ---------------------------------------------------------------------------
 // sub-panel LU in registers
 // ---------------------------------------------------------------------------
+// Candidate of a pivot search: |re| + |im| as the bits of a non-negative double, which
+// order like it (NaN counts as 0), and its row; INT_MAX: none.
+struct Pivot {
+  unsigned hi, lo;
+  int row;
+  // takes v of row r where it is larger; rows come in ascending order
+  __device__ __forceinline__ void offer(double2 v, int r) {
+    const double a = fabs(v.x) + fabs(v.y);
+    const unsigned h = a >= 0.0 ? (unsigned)__double2hiint(a) : 0u;
+    const unsigned l = a >= 0.0 ? (unsigned)__double2loint(a) : 0u;
+    if (row == INT_MAX || h > hi || (h == hi && l > lo)) {
+      hi = h;
+      lo = l;
+      row = r;
+    }
+  }
+  // lane of the warp's largest candidate, the lowest row among equals.  The upper
+  // words mostly decide; the lower words and rows are compared where they do not.
+  __device__ __forceinline__ int winner() const {
+    constexpr unsigned kAll = 0xffffffffu;
+    const unsigned h = __reduce_max_sync(kAll, hi);
+    unsigned m = __ballot_sync(kAll, hi == h);
+    if (m & (m - 1)) {  // the same for every lane
+      const unsigned l = __reduce_max_sync(kAll, hi == h ? lo : 0u);
+      const bool in = hi == h && lo == l;
+      const int r = __reduce_min_sync(kAll, in ? row : INT_MAX);
+      m = __ballot_sync(kAll, in && row == r);
+    }
+    return __ffs(m) - 1;
+  }
+};
+
 template <int W, int NW>
 struct PanelShared {
-  unsigned key[2][NW];
+  Pivot cand[2][NW];
   double2 prow[2][W], jrow[2][W];
   int swap[W];
 };
 
-// Candidate row r < 4096 of a pivot search as one word: the size |re| + |im| to 9
-// bits after the leading one (the upper word of a non-negative double orders like
-// it; NaN counts as 0), then the lowest row first.  A pivot is thus at least 0.998 of
-// the column's largest entry.
-__device__ __forceinline__ unsigned pivot_word(double2 v, int r) {
-  const double a = fabs(v.x) + fabs(v.y);
-  const unsigned key = a >= 0.0 ? (unsigned)__double2hiint(a) : 0u;
-  return (key << 1 & ~0xfffu) | (unsigned)(4095 - r);
-}
-// the same without a row, to 20 bits
-__device__ __forceinline__ unsigned pivot_key(double2 v) {
-  const double a = fabs(v.x) + fabs(v.y);
-  return a >= 0.0 ? (unsigned)__double2hiint(a) : 0u;
-}
 // neither zero nor NaN
 __device__ __forceinline__ bool pivot_ok(double2 v) { return fabs(v.x) + fabs(v.y) > 0.0; }
 
@@ -151,23 +169,22 @@ __device__ __forceinline__ double2 crecip(double2 v) {
 template <int W, int RPT, int T>
 __device__ __forceinline__ bool lu_columns(double2 (&a)[RPT][W], int w, int nrow, int t,
                                            PanelShared<W, T / 32> &s) {
-  static_assert(RPT * T <= 4096, "pivot_word holds 12 bits of row");
   const int lane = t & 31, warp = t >> 5;
   bool zero = false;
 #pragma unroll
   for (int j = 0; j < W; j++) {
     if (j < w) {
-      unsigned best = 0;
+      Pivot best{0u, 0u, INT_MAX};
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
         const int r = t + q * T;
-        if (r >= j && r < nrow) best = max(best, pivot_word(a[q][j], r));
+        if (r >= j && r < nrow) best.offer(a[q][j], r);
       }
-      const unsigned wm = __reduce_max_sync(0xffffffffu, best);
-      if (lane == 0) s.key[j & 1][warp] = wm;
+      if (lane == best.winner()) s.cand[j & 1][warp] = best;
       bar_rows<T>();
-      const unsigned bm = __reduce_max_sync(0xffffffffu, lane < T / 32 ? s.key[j & 1][lane] : 0u);
-      const int p = 4095 - (int)(bm & 0xfffu);
+      Pivot all{0u, 0u, INT_MAX};
+      if (lane < T / 32) all = s.cand[j & 1][lane];
+      const int p = __shfl_sync(0xffffffffu, all.row, all.winner());
       if (t == 0) s.swap[j] = p;
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
@@ -715,8 +732,7 @@ __global__ void __launch_bounds__(kPanelThreads)
                    double2 *__restrict__ work, int jb, int *__restrict__ swap,
                    int *__restrict__ info) {
   constexpr int T = kPanelThreads;
-  __shared__ unsigned key[T / 32];
-  __shared__ int idx[T / 32];
+  __shared__ Pivot cand[T / 32];
   __shared__ double2 u[sp::kNb];
   __shared__ double2 D[sp::kNb][sp::kNb + 1];
   __shared__ double2 buf[2][2][sp::kNb], dinv[2][sp::kNb];
@@ -730,26 +746,13 @@ __global__ void __launch_bounds__(kPanelThreads)
   bool zero = false;
   for (int j = 0; j < nb; j++) {
     double2 *col = F + (jb + j) * n;
-    unsigned best = 0;
-    int bi = INT_MAX;
-    for (int r = jb + j + tid; r < k; r += T) {
-      const unsigned kv = pivot_key(col[r]);
-      if (bi == INT_MAX || kv > best) {
-        best = kv;
-        bi = r;
-      }
-    }
-    const unsigned wm = __reduce_max_sync(0xffffffffu, bi == INT_MAX ? 0u : best);
-    const int wi = __reduce_min_sync(0xffffffffu, best == wm ? bi : INT_MAX);
-    if (lane == 0) {
-      key[warp] = wm;
-      idx[warp] = wi;
-    }
+    Pivot best{0u, 0u, INT_MAX};
+    for (int r = jb + j + tid; r < k; r += T) best.offer(col[r], r);
+    if (lane == best.winner()) cand[warp] = best;
     __syncthreads();
-    const unsigned ck = lane < T / 32 ? key[lane] : 0u;
-    const int ci = lane < T / 32 ? idx[lane] : INT_MAX;
-    const unsigned bm = __reduce_max_sync(0xffffffffu, ci == INT_MAX ? 0u : ck);
-    const int p = __reduce_min_sync(0xffffffffu, ck == bm ? ci : INT_MAX);
+    Pivot all{0u, 0u, INT_MAX};
+    if (lane < T / 32) all = cand[lane];
+    const int p = __shfl_sync(0xffffffffu, all.row, all.winner());
     if (tid == 0) swap[f.own0 + jb + j] = p;
     if (tid < nb) {
       double2 *c = F + (jb + tid) * n;
