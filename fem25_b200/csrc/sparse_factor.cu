@@ -155,11 +155,14 @@ __device__ __forceinline__ void bar_rows() {
   asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
 }
 
-// 1 / v, zero when v is no pivot
+// 1 / v, zero when v is no pivot; scaled by a power of two around |v|, so that |v|^2
+// neither under- nor overflows
 __device__ __forceinline__ double2 crecip(double2 v) {
   if (!pivot_ok(v)) return make_double2(0.0, 0.0);
-  const double d = 1.0 / (v.x * v.x + v.y * v.y);
-  return make_double2(v.x * d, -v.y * d);
+  const int e = (__double2hiint(fmax(fabs(v.x), fabs(v.y))) >> 20) - 1023;
+  const double f = __hiloint2double((1023 - max(-1021, min(1021, e))) << 20, 0);
+  const double x = f * v.x, y = f * v.y, d = 1.0 / (x * x + y * y);
+  return make_double2(x * d * f, -y * d * f);
 }
 
 // LU with partial pivoting of the w <= W columns a[q][0..w) of rows

@@ -1,11 +1,18 @@
-"""Pivots of the sparse factorisation: their choice.  Beside ones on the diagonal, every node's first two DOFs p < q hold
+"""Pivots of the sparse factorisation.
+
+Choice: beside ones on the diagonal, every node's first two DOFs p < q hold
   [ 1      2^60 ]
   [ 1 + d  1    ]
 whose partial pivoting must take row q.  Then x_p = (b_q - x_q) / (1 + d) loses
 nothing; with row p as the pivot x_p is b_p - 2^60 x_q and wrong by about 2^7.  For
 |x| < 2 the right order leaves a handful of roundings of numbers below 5, so 2e-14
 bounds the error.  d from 2^-12 to 2^-40, in fronts of every kernel of the
-factorisation (the small ones, and the larger ones at each sub-panel width)."""
+factorisation (the small ones, and the larger ones at each sub-panel width).
+
+Range: powers of two scale the matrix and the right-hand side until the squares of
+the entries under- or overflow, where 1 / pivot is still a normal number.  Scaling by a
+power of two is exact, so only the order of the solve's sums differs from the unscaled
+solution: 1e-9 relative leaves two orders above the known-field errors of such meshes."""
 import numpy as np
 import pytest
 
@@ -49,3 +56,21 @@ def test_pivot_choice(case, width, bits, monkeypatch):
     d = torch.from_numpy(b[None]).cuda()
     ctx.sparse_solve(d, 0)
     assert np.abs(d.cpu().numpy()[0] - x).max() <= 2e-14
+
+
+@pytest.mark.parametrize("exponent", [-560, -520, 520])
+@pytest.mark.parametrize("width", [8, 1])
+def test_pivot_range(case, width, exponent, monkeypatch):
+    monkeypatch.setenv("FEM25_PANEL_WIDTH", str(width))
+    ctx, g, pairs = case
+    a = torch.zeros(g.nzero, dtype=torch.complex128, device="cuda:0")
+    ctx.assemble("B", *pairs[70], a)
+    rng = np.random.default_rng(5)
+    b = torch.from_numpy(rng.standard_normal((1, g.ndof)) + 1j * rng.standard_normal((1, g.ndof))).cuda()
+    scale = 2.0 ** (exponent - int(np.log2(float(a.abs().max()))))  # exponent: of the largest entry
+    want, got = b.clone(), b * scale
+    ctx.sparse_factor(a)
+    ctx.sparse_solve(want, 0)
+    ctx.sparse_factor(a * scale)
+    ctx.sparse_solve(got, 0)
+    assert float(torch.linalg.norm(got - want) / torch.linalg.norm(want)) <= 1e-9
