@@ -97,8 +97,8 @@ void free_ctx(Ctx *c) {
                   c->d_elem_wts, c->d_fmat, c->d_cadj_col0, c->d_cadj_pair_col, c->d_cadj_pair_elem,
                   c->d_cadj_dptr, c->d_cadj_dent, c->d_cadj_w, c->d_nonpml, c->d_cdist, c->d_prim, c->d_desc,
                   c->d_tc_tab, c->d_qp, c->d_qs, c->d_cov, c->d_cov_ops, c->d_cov_opptr,
-                  c->d_cov_tx, c->d_cov_node, c->d_cov_exps, c->d_maskg, c->d_avg_work, c->d_post_mrdof,
-                  c->d_post_bits, c->d_hvec, c->d_hgrad, c->d_call, c->d_tasks, c->d_tasks_pml};
+                  c->d_cov_tx, c->d_cov_node, c->d_cov_exps, c->d_maskg, c->d_avg_work, c->d_hvec,
+                  c->d_hgrad, c->d_tasks, c->d_tasks_pml};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &e : c->ev)
@@ -110,17 +110,23 @@ void free_ctx(Ctx *c) {
   if (c->copy_st) cudaStreamDestroy(c->copy_st);
   for (auto &s : c->elem_st)
     if (s) cudaStreamDestroy(s);
+  for (auto &b : c->call_blocks) cudaFree(b.second);
+  c->post_tab.reset();
   free_dense(c);
   free_sparse(c);
 }
 
-// The arrays of one host-array call in the context's device block, copied by the
-// driver from and to the caller's memory: four to seven cudaMalloc and cudaFree a
-// call made the post-solve call 1.1 ms for 64 sources x 190 receivers, 0.27 ms with
-// the block kept (the kernel itself 0.14 -> 0.09).
+// The arrays of one host-array call in a device block of its own, copied by the driver
+// from and to the caller's memory.  The call ends synchronised and hands its block back
+// to the context, which keeps up to kCallKeep bytes of them: four to seven cudaMalloc and
+// cudaFree a call made the post-solve call 1.1 ms for 64 sources x 190 receivers, 0.27 ms
+// without them (the kernel itself 0.14 -> 0.09).  cudaMallocAsync from a pool of the
+// context's that keeps as much took 1.2 ms.
+constexpr size_t kCallKeep = 16u << 20;
 struct CallBuffers {
   Ctx *c;
   cudaStream_t st;
+  std::pair<size_t, char *> block{0, nullptr};
   size_t used = 0;
   struct Arr {
     size_t off, bytes;
@@ -129,6 +135,19 @@ struct CallBuffers {
   };
   std::vector<Arr> arr;
   CallBuffers(Ctx *ctx, cudaStream_t s) : c(ctx), st(s) {}
+  ~CallBuffers() {
+    if (!block.second) return;
+    {
+      std::lock_guard<std::mutex> lock(c->call_mu);
+      size_t kept = block.first;
+      for (const auto &b : c->call_blocks) kept += b.first;
+      if (kept <= kCallKeep) {
+        c->call_blocks.push_back(block);
+        return;
+      }
+    }
+    cudaFree(block.second);
+  }
   // adds an input (src) or output (dst); returns its index
   int add(size_t bytes, const void *src, void *dst) {
     arr.push_back({used, bytes, src, dst});
@@ -137,19 +156,38 @@ struct CallBuffers {
   }
   template <class T>
   T *dev(int i) const {
-    return reinterpret_cast<T *>(c->d_call + arr[i].off);
+    return reinterpret_cast<T *>(block.second + arr[i].off);
+  }
+  // the smallest kept block that holds the arrays; where none does, the largest makes way
+  // for a new one
+  cudaError_t take() {
+    std::pair<size_t, char *> small{0, nullptr};
+    {
+      std::lock_guard<std::mutex> lock(c->call_mu);
+      auto &v = c->call_blocks;
+      std::sort(v.begin(), v.end());
+      auto it = std::lower_bound(v.begin(), v.end(), std::make_pair(used, (char *)nullptr));
+      if (it != v.end()) {
+        block = *it;
+        v.erase(it);
+        return cudaSuccess;
+      }
+      if (!v.empty()) {
+        small = v.back();
+        v.pop_back();
+      }
+    }
+    if (small.second) cudaFree(small.second);
+    cudaError_t e = cudaMalloc(&block.second, used);
+    if (e) block.second = nullptr;
+    else block.first = used;
+    return e;
   }
   cudaError_t upload() {
-    cudaError_t e;
-    if (used > c->d_call_bytes) {
-      if (c->d_call) cudaFree(c->d_call);
-      c->d_call = nullptr;
-      c->d_call_bytes = 0;
-      if ((e = cudaMalloc(&c->d_call, used))) return e;
-      c->d_call_bytes = used;
-    }
+    cudaError_t e = take();
+    if (e) return e;
     for (const Arr &a : arr)
-      if (a.src && (e = cudaMemcpyAsync(c->d_call + a.off, a.src, a.bytes, cudaMemcpyHostToDevice, st)))
+      if (a.src && (e = cudaMemcpyAsync(block.second + a.off, a.src, a.bytes, cudaMemcpyHostToDevice, st)))
         return e;
     return cudaSuccess;
   }
@@ -157,11 +195,38 @@ struct CallBuffers {
   cudaError_t download() {
     cudaError_t e;
     for (const Arr &a : arr)
-      if (a.dst && (e = cudaMemcpyAsync(a.dst, c->d_call + a.off, a.bytes, cudaMemcpyDeviceToHost, st)))
+      if (a.dst && (e = cudaMemcpyAsync(a.dst, block.second + a.off, a.bytes, cudaMemcpyDeviceToHost, st)))
         return e;
     return cudaStreamSynchronize(st);
   }
 };
+
+// Receiver tables for MRDOF: the context's where it repeats, else made for it and kept.
+// Returns once they are on the device.
+cudaError_t receiver_table(Ctx *c, int nrec, const int *mrdof, cudaStream_t st,
+                           std::shared_ptr<const RecvTable> *out) {
+  const size_t n = 3 * (size_t)nrec;
+  std::lock_guard<std::mutex> lock(c->call_mu);
+  *out = c->post_tab;
+  if (*out && (*out)->mrdof.size() == n && std::equal(mrdof, mrdof + n, (*out)->mrdof.begin()))
+    return cudaSuccess;
+  auto t = std::make_shared<RecvTable>();
+  t->mrdof.assign(mrdof, mrdof + n);
+  std::vector<uint32_t> bits(((size_t)c->ndof + 31) / 32, 0u);
+  for (size_t k = 0; k < n; k++)
+    if (mrdof[k] > 0) bits[(mrdof[k] - 1) >> 5] |= 1u << ((mrdof[k] - 1) & 31);
+  cudaError_t e;
+  if ((e = cudaMalloc(&t->d_mrdof, sizeof(int) * n)) ||
+      (e = cudaMalloc(&t->d_bits, sizeof(uint32_t) * bits.size())) ||
+      (e = cudaMemcpyAsync(t->d_mrdof, mrdof, sizeof(int) * n, cudaMemcpyHostToDevice, st)) ||
+      (e = cudaMemcpyAsync(t->d_bits, bits.data(), sizeof(uint32_t) * bits.size(),
+                           cudaMemcpyHostToDevice, st)) ||
+      (e = cudaStreamSynchronize(st)))
+    return e;
+  c->post_tab = t;
+  *out = t;
+  return cudaSuccess;
+}
 
 int read_err_word(Ctx *c, cudaStream_t st) {
   int h = 0;
@@ -1110,22 +1175,8 @@ int fem25_postsolve_dev(fem25_ctx *h, int nsrc, int nrec, const int *mrdof, cons
   }
   CK(cudaSetDevice(c->device), "set device");
   cudaStream_t st = (cudaStream_t)stream;
-  // receiver tables: rebuilt only when MRDOF differs from the last call's
-  if (c->post_mrdof.size() != 3 * (size_t)nrec ||
-      !std::equal(c->post_mrdof.begin(), c->post_mrdof.end(), mrdof)) {
-    CK(cudaStreamSynchronize(st), "synchronize");
-    if (c->d_post_mrdof) cudaFree(c->d_post_mrdof);
-    if (c->d_post_bits) cudaFree(c->d_post_bits);
-    c->d_post_mrdof = nullptr;
-    c->d_post_bits = nullptr;
-    c->post_mrdof.clear();
-    std::vector<uint32_t> bits(((size_t)c->ndof + 31) / 32, 0u);
-    for (int k = 0; k < 3 * nrec; k++)
-      if (mrdof[k] > 0) bits[(mrdof[k] - 1) >> 5] |= 1u << ((mrdof[k] - 1) & 31);
-    CK(dalloc_copy(&c->d_post_mrdof, mrdof, 3 * (size_t)nrec), "postsolve");
-    CK(dalloc_copy(&c->d_post_bits, bits.data(), bits.size()), "postsolve");
-    c->post_mrdof.assign(mrdof, mrdof + 3 * (size_t)nrec);
-  }
+  std::shared_ptr<const RecvTable> tab;
+  CK(receiver_table(c, nrec, mrdof, st, &tab), "postsolve");
   const double omega = 6.2831853071795862 * freq;
   std::vector<float> trig(4 * (size_t)nrec);
   for (int ir = 0; ir < nrec; ir++) {
@@ -1146,7 +1197,7 @@ int fem25_postsolve_dev(fem25_ctx *h, int nsrc, int nrec, const int *mrdof, cons
   const int mi = b.add(sizeof(float) * nsrc, nullptr, misfit);
   auto run = [&]() -> int {
     CK(b.upload(), "postsolve");
-    CK(launch_postsolve(c, nsrc, nrec, c->d_post_mrdof, c->d_post_bits, b.dev<float>(t), freq, azmod,
+    CK(launch_postsolve(c, nsrc, nrec, tab->d_mrdof, tab->d_bits, b.dev<float>(t), freq, azmod,
                         b.dev<float>(rv), ue, sol, b.dev<float>(ob), b.dev<float>(w),
                         b.dev<float>(es), rhs, b.dev<float>(mi), st),
        "postsolve");

@@ -5,7 +5,10 @@
 
 #include <cstdint>
 
+#include <memory>
+#include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "fem25_internal.h"
@@ -73,6 +76,18 @@ struct ShapeTabs {
   double d[kNint][kNl];
 };
 ShapeTabs shape_tables(const Tables &t);
+
+// Receiver tables on the device for one MRDOF: the receiver DOFs as a bitmap (one bit
+// per DOF) and MRDOF itself
+struct RecvTable {
+  std::vector<int> mrdof;
+  int *d_mrdof = nullptr;
+  uint32_t *d_bits = nullptr;
+  ~RecvTable() {
+    if (d_mrdof) cudaFree(d_mrdof);
+    if (d_bits) cudaFree(d_bits);
+  }
+};
 
 // Options of the misfit / adjoint source (the reference's INV_INFO fields
 // NORM, IRESTP, IBPHASE, the thresholds of COBJ4 and the DTMAX phase-jump
@@ -186,19 +201,18 @@ struct Ctx {
   // (0: the default, about half a second) and the time-out test hook
   long long wait_limit = 0;
   int wait_inject = 0;
-  // receiver tables of the fused post-solve pass, kept while MRDOF repeats:
-  // the receiver DOFs as a bitmap (one bit per DOF) and MRDOF itself
-  std::vector<int> post_mrdof;
-  int *d_post_mrdof = nullptr;
-  uint32_t *d_post_bits = nullptr;
+  // receiver tables of the fused post-solve pass, kept while MRDOF repeats; a call
+  // holds a reference to those that it uses
+  std::shared_ptr<const RecvTable> post_tab;
   // device scratch of the host-buffer drop-ins (fem25_asmb_peff,
   // fem25_cfmat_adjgrad): 3 COMPLEX*8 [NDOF] vectors and GRADL
   float2 *d_hvec = nullptr;
   float *d_hgrad = nullptr;
-  // device block of the host-array calls fem25_misfit_dev / fem25_postsolve_dev,
-  // which return after their stream is done; grown to the largest call
-  char *d_call = nullptr;
-  size_t d_call_bytes = 0;
+  // device blocks of the host-array calls fem25_misfit_dev / fem25_postsolve_dev that no
+  // call is using, as (bytes, address): each call takes one of its own, so that calls of
+  // several threads may overlap
+  std::vector<std::pair<size_t, char *>> call_blocks;
+  std::mutex call_mu;  // of post_tab and call_blocks
   // misfit options (fem25_misfit_options); the defaults of the reference
   MisfitOpts mopt{2, 3, 0, 0.0f, 0.0f, 0.0f, 0.0f, 0.0, {1.0f, 0.0f}};
   // optional CUDA-event timing of the dominant kernels

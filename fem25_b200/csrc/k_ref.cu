@@ -451,8 +451,10 @@ cudaError_t launch_postsolve(Ctx *c, int nsrc, int nrec, const int *d_mrdof, con
   float th = (float)azmod * 0.017453292519943295f;
   float4 rot = make_float4(cosf(th), sinf(th), cosf(-th), sinf(-th));
   const size_t smem = sizeof(float) * 3 * (size_t)nrec;
+  // the same limit in every call: one for this call's size could be lowered by another
+  // thread's before the launch
   cudaError_t e = cudaFuncSetAttribute(k_postsolve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)std::max(smem, (size_t)1));
+                                       (int)sizeof(float) * 3 * FEM25_POSTSOLVE_MAX_REC);
   if (e != cudaSuccess) return e;
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);

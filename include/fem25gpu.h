@@ -11,7 +11,9 @@
  *   - index arrays hold Fortran 1-based values (IENG, LM, IRPTR, JCPTR ...)
  *     and two-dimensional arrays keep their Fortran column-major layout;
  *   - buffers belong to the caller; complex values are interleaved (re, im).
- * A context is not re-entrant; several contexts may run on separate streams.
+ * A context is not re-entrant, except that several threads may be in fem25_misfit_dev
+ * and fem25_postsolve_dev with arrays and streams of their own; several contexts may
+ * run on separate streams.
  * `stream` arguments are cudaStream_t values passed as void* (NULL = default).
  */
 #ifndef FEM25GPU_H
