@@ -668,15 +668,12 @@ int fem25_assemble_dev(fem25_ctx *h, char cftype, double freq, double py, double
   return FEM25_OK;
 }
 
-int fem25_asmble_driver(fem25_ctx *h, int nzloc, char cftype, double freq, double py,
-                        float *cdist) {
-  if (!h || !cdist) return FEM25_ERR_ARG;
-  Ctx *c = &h->c;
-  if ((long long)nzloc != c->nzero) return fail(c, FEM25_ERR_ARG, "asmble_driver: NZLOC != NZERO");
-  if (cftype != 'S' && cftype != 'B')
-    return fail(c, FEM25_ERR_ARG, "asmble_driver: CFTYPE must be 'S' or 'B'");
-  if (!(freq > 0.0)) return fail(c, FEM25_ERR_ARG, "asmble_driver: FREQ must be > 0");
-  CK(cudaSetDevice(c->device), "set device");
+}  // extern "C"
+
+namespace {
+
+// The launches and copies of fem25_asmble_driver
+int asmble_driver(Ctx *c, int nzloc, char cftype, double freq, double py, float *cdist) {
   int r = ensure_plain(c, nullptr);
   if (r) return r;
   if (!c->d_cdist) CK(cudaMalloc(&c->d_cdist, sizeof(float2) * (size_t)nzloc), "cdist buffer");
@@ -714,6 +711,26 @@ int fem25_asmble_driver(fem25_ctx *h, int nzloc, char cftype, double freq, doubl
   // a last chunk without rows of its own has no copy behind it
   for (cudaStream_t s : c->elem_st) CK(cudaStreamSynchronize(s), "element streams");
   return read_err_word(c, 0);
+}
+
+}  // namespace
+
+extern "C" {
+
+int fem25_asmble_driver(fem25_ctx *h, int nzloc, char cftype, double freq, double py,
+                        float *cdist) {
+  if (!h || !cdist) return FEM25_ERR_ARG;
+  Ctx *c = &h->c;
+  if ((long long)nzloc != c->nzero) return fail(c, FEM25_ERR_ARG, "asmble_driver: NZLOC != NZERO");
+  if (cftype != 'S' && cftype != 'B')
+    return fail(c, FEM25_ERR_ARG, "asmble_driver: CFTYPE must be 'S' or 'B'");
+  if (!(freq > 0.0)) return fail(c, FEM25_ERR_ARG, "asmble_driver: FREQ must be > 0");
+  CK(cudaSetDevice(c->device), "set device");
+  const int r = asmble_driver(c, nzloc, cftype, freq, py, cdist);
+  if (r)  // nothing of this call outlives it, the copies into cdist above all
+    for (cudaStream_t s : {c->elem_st[0], c->elem_st[1], c->copy_st, (cudaStream_t) nullptr})
+      cudaStreamSynchronize(s);
+  return r;
 }
 
 int fem25_assemble_batch_dev(fem25_ctx *h, int n, const char *cftype, const double *freq,

@@ -1018,7 +1018,7 @@ static cudaError_t sparse_solve_attributes() {
                               (int)(row * (sp::kSmallK + kChunk)));
 }
 
-int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *msg) {
+static int sparse_factor_run(Ctx *c, const double *csr128, cudaStream_t st, std::string *msg) {
   if (!c->sparse) c->sparse = new SparseLU();
   SparseLU *s = c->sparse;
   s->factored = false;
@@ -1077,6 +1077,17 @@ int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *ms
   }
   s->factored = true;
   return 0;
+}
+
+int sparse_factor(Ctx *c, const double *csr128, cudaStream_t st, std::string *msg) {
+  const int r = sparse_factor_run(c, csr128, st, msg);
+  if (r) {  // nothing of this call outlives it: a level may have stopped between its streams
+    for (int g = 0; g < sp::kStreams; g++)
+      for (cudaStream_t q : {c->sparse->st[g], c->sparse->side[g]})
+        if (q) cudaStreamSynchronize(q);
+    cudaStreamSynchronize(st);
+  }
+  return r;
 }
 
 // One level's launches of a pass, 8 NT right-hand sides a CTA
