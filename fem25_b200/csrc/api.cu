@@ -312,31 +312,34 @@ int ensure_batch(Ctx *c, cudaStream_t st) {
 // the last element holding DOF r (GENID numbers DOFs in element order, so
 // rows complete nearly in order) has been computed.
 int ensure_driver_plan(Ctx *c) {
-  if (c->copy_st) return FEM25_OK;
   const int nch = std::max(1, std::min(16, c->nelem / 148));
-  std::vector<int> last(c->ndof, -1);
-  for (int e = 0; e < c->nelem; e++)
-    for (int k = 0; k < 3 * kNen; k++) {
-      const int d = c->h_lm[(size_t)e * 3 * kNen + k];
-      if (d > 0) last[d - 1] = e;
+  if (c->drv_elem.empty()) {
+    std::vector<int> last(c->ndof, -1);
+    for (int e = 0; e < c->nelem; e++)
+      for (int k = 0; k < 3 * kNen; k++) {
+        const int d = c->h_lm[(size_t)e * 3 * kNen + k];
+        if (d > 0) last[d - 1] = e;
+      }
+    std::vector<int> elem(nch + 1, 0), row(nch + 1, 0);
+    for (int k = 0; k <= nch; k++) elem[k] = (int)((long long)k * c->nelem / nch);
+    int r = 0;
+    for (int k = 1; k <= nch; k++) {
+      while (r < c->ndof && last[r] < elem[k]) r++;
+      row[k] = r;
     }
-  c->drv_elem.assign(nch + 1, 0);
-  c->drv_row.assign(nch + 1, 0);
-  for (int k = 0; k <= nch; k++) c->drv_elem[k] = (int)((long long)k * c->nelem / nch);
-  int r = 0;
-  for (int k = 1; k <= nch; k++) {
-    while (r < c->ndof && last[r] < c->drv_elem[k]) r++;
-    c->drv_row[k] = r;
+    if (row[nch] != c->ndof)
+      return fail(c, FEM25_ERR_PATTERN, "asmble_driver: DOF outside every element");
+    c->drv_elem = elem;
+    c->drv_row = row;
   }
-  if (c->drv_row[nch] != c->ndof)
-    return fail(c, FEM25_ERR_PATTERN, "asmble_driver: DOF outside every element");
-  c->drv_ev.assign(nch, nullptr);
-  for (auto &e : c->drv_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-  c->drv_elem_ev.assign(nch + 1, nullptr);
-  for (auto &e : c->drv_elem_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-  for (auto &s : c->elem_st)
-    CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "element streams");
-  CK(cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking), "copy stream");
+  // each by itself: a call after one that failed makes what is missing
+  c->drv_ev.resize(nch, nullptr);
+  c->drv_elem_ev.resize(nch + 1, nullptr);
+  for (auto *v : {&c->drv_ev, &c->drv_elem_ev})
+    for (auto &e : *v)
+      if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+  for (cudaStream_t *s : {&c->elem_st[0], &c->elem_st[1], &c->copy_st})
+    if (!*s) CK(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking), "driver streams");
   return FEM25_OK;
 }
 

@@ -1036,20 +1036,26 @@ static int sparse_factor_run(Ctx *c, const double *csr128, cudaStream_t st, std:
   SPCK(sparse_solve_attributes<1>(), "kernel attributes");
   SPCK(sparse_solve_attributes<2>(), "kernel attributes");
   SPCK(sparse_solve_attributes<4>(), "kernel attributes");
+  // streams, events and buffers each by itself: a call after one that failed makes what
+  // is missing
   if (!s->ready) {
     // the groups' own streams go before their side streams: a panel must not queue
     // behind the update beside it
     int least = 0, greatest = 0;
     SPCK(cudaDeviceGetStreamPriorityRange(&least, &greatest), "streams");
+    auto stream = [](cudaStream_t *q, int priority) {
+      return *q ? cudaSuccess : cudaStreamCreateWithPriority(q, cudaStreamNonBlocking, priority);
+    };
+    auto event = [](cudaEvent_t *q) {
+      return *q ? cudaSuccess : cudaEventCreateWithFlags(q, cudaEventDisableTiming);
+    };
     for (int g = 0; g < sp::kStreams; g++) {
-      SPCK(cudaStreamCreateWithPriority(&s->st[g], cudaStreamNonBlocking, greatest), "streams");
-      SPCK(cudaStreamCreateWithPriority(&s->side[g], cudaStreamNonBlocking, least), "streams");
-      for (cudaEvent_t *q : {&s->done[g], &s->applied[g], &s->updated[g]})
-        SPCK(cudaEventCreateWithFlags(q, cudaEventDisableTiming), "events");
+      SPCK(stream(&s->st[g], greatest), "streams");
+      SPCK(stream(&s->side[g], least), "streams");
+      for (cudaEvent_t *q : {&s->done[g], &s->applied[g], &s->updated[g]}) SPCK(event(q), "events");
     }
-    SPCK(cudaEventCreateWithFlags(&s->ready, cudaEventDisableTiming), "events");
+    SPCK(event(&s->ready), "events");
   }
-  // each by itself: a call after one that ran out of memory makes what is missing
   auto keep = [](auto **p, size_t n) {
     return *p ? cudaSuccess : cudaMalloc(p, sizeof(**p) * std::max(n, (size_t)1));
   };

@@ -1,7 +1,8 @@
 """Calls that spread their work over streams of the context, when a CUDA call inside
 them fails: the library's objects linked against a fake runtime (fake_cudart.cpp)
 that runs no kernels and fails its n-th call.  Wherever the call stops it leaves no
-work that nobody has waited for, and the next call succeeds."""
+work that nobody has waited for, the next call succeeds, and the context's streams
+and events are made once and destroyed with it."""
 import os
 import subprocess
 import sys
@@ -40,7 +41,9 @@ while True:  # the first failures come in a context that has made nothing yet
 fake.fake_fail_at(0)
 assert failed > 20, failed
 assert call() == 0 and fake.fake_pending() == 0
+made = [fake.fake_live(k) for k in (0, 1)]
 ctx.close()
+assert [fake.fake_live(k) for k in (0, 1)] == [0, 0], (made, [fake.fake_live(k) for k in (0, 1)])
 """
 
 
