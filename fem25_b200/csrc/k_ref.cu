@@ -496,14 +496,18 @@ cudaError_t launch_misfit_part(Ctx *c, int nsrc, int nrec, const int *d_mrdof, c
 // threads form FORCEV(row) += CARG * WAVE * CWGHT in IQE order
 // (vforce25.f:326-330).
 // Bound: FP64 operations, rounded one by one.  A thread takes node b = t % 25
-// with the five nodes a = 5 (t / 25) + i: the 17 products that depend on b alone
-// serve five pairs (52 operations a pair and point beside them, 68 before), and
-// 81 KB of shared memory (CARG takes the place of the shape derivatives) let two
+// with the A nodes a = A (t / 25) + i.  A = 5: the 17 products that depend on b
+// alone serve five pairs (52 operations a pair and point beside them, 68 before),
+// and 81 KB of shared memory (CARG takes the place of the shape derivatives) let two
 // CTAs share an SM, one summing while the other prepares.  11 000 anchors:
-// 5.1 ms against 7.2 ms with one pair a thread and one CTA of 640 an SM.
+// 5.1 ms against 7.2 ms with one pair a thread and one CTA of 640 an SM.  A = 1,
+// 640 threads, for at most one anchor an SM, where the length of one CTA counts:
+// 64, 108 and 143 anchors 140, 145 and 150 us against 158, 164 and 168 with A = 5;
+// 154 anchors 242 (the earlier kernel, the same layout) against 203.
 // ---------------------------------------------------------------------------
 constexpr int kRefThreads = 640;
-constexpr int kCfThreads = 128, kCfA = 5;
+// threads for A node pairs each, in whole warps
+constexpr int cf_threads(int A) { return (kNab / A + 31) / 32 * 32; }
 constexpr int kCfQc = 13;  // geometry 0-4, then the operator's point coefficients
 constexpr int kCfSm = 2 * kNq * kNen + kCfQc * kNq;
 
@@ -512,12 +516,14 @@ struct RefArgs {
   int lisp, accumulate, ncon, nnpg;
 };
 
-__global__ void __launch_bounds__(kCfThreads, 2)
+template <int A>
+__global__ void __launch_bounds__(cf_threads(A), A == 1 ? 1 : 2)
     k_ref_cfmat(MeshView mv, DevTables dt, RefArgs ra, const int *__restrict__ lm,
                 const int *__restrict__ anchor_of_col, const int *__restrict__ mconn,
                 const double *__restrict__ elem_wts, const int *__restrict__ jcsc,
                 const int *__restrict__ icsc, const float2 *__restrict__ wave,
                 float2 *__restrict__ fmat, int *__restrict__ err) {
+  constexpr int kThreads = cf_threads(A);
   extern __shared__ double sm[];
   double *shx = sm, *shz = sm + kNq * kNen;
   double *qc = sm + 2 * kNq * kNen;             // [kNq][kCfQc]
@@ -528,7 +534,7 @@ __global__ void __launch_bounds__(kCfThreads, 2)
   const int p = anchor_of_col[col];  // 0-based anchor (INPG-1)
   const int i1 = jcsc[col] - 1, i2 = jcsc[col + 1] - 1, nnzrow = i2 - i1;
   float2 *forcev = fmat + i1;
-  for (int k = t; k < nnzrow; k += kCfThreads) forcev[k] = make_float2(0.0f, 0.0f);
+  for (int k = t; k < nnzrow; k += kThreads) forcev[k] = make_float2(0.0f, 0.0f);
   // elements of the anchor, in MCONN order; without accumulation only the
   // last one leaves a trace in FORCEV
   int elist[8], ne = 0;
@@ -543,12 +549,12 @@ __global__ void __launch_bounds__(kCfThreads, 2)
   for (int ie_ = first; ie_ < ne; ie_++) {
     const int e = elist[ie_];
     const int4 ie = mv.ieng[e];
-    for (int k = t; k < kNee; k += kCfThreads) {
+    for (int k = t; k < kNee; k += kThreads) {
       const int d = lm[(size_t)e * kNee + k];
       dof[k] = d;
       wv[k] = d > 0 ? wave[d - 1] : make_float2(0.0f, 0.0f);
     }
-    for (int q = t; q < kNq; q += kCfThreads) {
+    for (int q = t; q < kNq; q += kThreads) {
       const int intx = q % kNint, intz = q / kNint;
       QGeo g;
       if (!quad_geo(mv, dt, ie, q, false, g)) atomicCAS(err, 0, e + 1);
@@ -588,7 +594,7 @@ __global__ void __launch_bounds__(kCfThreads, 2)
     }
     __syncthreads();
 #pragma unroll 4
-    for (int idx = t; idx < kNq * kNen; idx += kCfThreads) {
+    for (int idx = t; idx < kNq * kNen; idx += kThreads) {
       const double *c = qc + kCfQc * (idx / kNen);
       const double *sl = dt.shl + 3 * (size_t)idx;
       const double drnxi = sl[0], drneta = sl[1];
@@ -596,12 +602,12 @@ __global__ void __launch_bounds__(kCfThreads, 2)
       shz[idx] = -(drnxi * c[1] - drneta * c[0]) / c[4];
     }
     __syncthreads();
-    const bool on = t < kNen * kNl;
-    const int a0 = kCfA * (t / kNen), b = t % kNen;
-    double m0[kCfA], m1[kCfA], r00[kCfA], r11[kCfA], r22[kCfA], r02[kCfA], r20[kCfA];
-    double r01[kCfA], r10[kCfA], r12[kCfA], r21[kCfA];
+    const bool on = t < kNab / A;
+    const int a0 = A * (t / kNen), b = t % kNen;
+    double m0[A], m1[A], r00[A], r11[A], r22[A], r02[A], r20[A];
+    double r01[A], r10[A], r12[A], r21[A];
 #pragma unroll
-    for (int i = 0; i < kCfA; i++)
+    for (int i = 0; i < A; i++)
       m0[i] = m1[i] = r00[i] = r11[i] = r22[i] = r02[i] = r20[i] = r01[i] = r10[i] = r12[i] =
           r21[i] = 0.0;
     if (on) {
@@ -621,7 +627,7 @@ __global__ void __launch_bounds__(kCfThreads, 2)
           const double m2n = m2ws * phib, m2wx = m2ws * phibx, m2wz = m2ws * phibz;
           const double mwn = mws * phib, mwx = mws * phibx, mwz = mws * phibz;
 #pragma unroll
-          for (int i = 0; i < kCfA; i++) {
+          for (int i = 0; i < A; i++) {
             const int a = q * kNen + a0 + i;
             const double phia = __ldg(dt.shn + a), phiax = shx[a], phiaz = shz[a];
             m0[i] = m0[i] + rm1n * phia;  // DME(1,1) = DME(3,3)
@@ -641,7 +647,7 @@ __global__ void __launch_bounds__(kCfThreads, 2)
     __syncthreads();  // every read of the shape derivatives is done
     if (on) {
 #pragma unroll
-      for (int i = 0; i < kCfA; i++) {
+      for (int i = 0; i < A; i++) {
         float *row0 = carg + (3 * (a0 + i)) * kNee + 3 * b, *row1 = row0 + kNee, *row2 = row1 + kNee;
         row0[0] = __double2float_rn(m0[i] + r00[i]);
         row0[1] = __double2float_rn(0.0 + r01[i]);
@@ -655,7 +661,7 @@ __global__ void __launch_bounds__(kCfThreads, 2)
       }
     }
     if (!ra.accumulate)
-      for (int k = t; k < nnzrow; k += kCfThreads) forcev[k] = make_float2(0.0f, 0.0f);
+      for (int k = t; k < nnzrow; k += kThreads) forcev[k] = make_float2(0.0f, 0.0f);
     __syncthreads();
     if (t < kNee) {
       const int ipe = t;
@@ -1208,6 +1214,18 @@ __global__ void k_ref_adjflam(int ncol, const int *__restrict__ jcsc, const int 
   gradl[k] = gradl[k] + (-1.0f) * v;
 }
 
+template <int A>
+static cudaError_t ref_cfmat(Ctx *c, const RefArgs &ra, const float *wave, cudaStream_t st) {
+  constexpr size_t smem = sizeof(double) * kCfSm;
+  cudaError_t e = cudaFuncSetAttribute(k_ref_cfmat<A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem);
+  if (e) return e;
+  k_ref_cfmat<A><<<c->rg.nnpinv, cf_threads(A), smem, st>>>(
+      c->mv, c->dt, ra, c->d_lm, c->d_rg_anchor, c->d_mconn, c->d_elem_wts, c->d_jcsc, c->d_icsc,
+      (const float2 *)wave, c->d_fmat, c->d_err);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_ref_cfmat(Ctx *c, int lisp, double vpvs, double omega, double py,
                              const float *wave, int accumulate, cudaStream_t st) {
   RefArgs ra;
@@ -1218,13 +1236,10 @@ cudaError_t launch_ref_cfmat(Ctx *c, int lisp, double vpvs, double omega, double
   ra.accumulate = accumulate;
   ra.ncon = c->rg.ncon;
   ra.nnpg = c->nnpg;
-  cudaError_t e = cudaFuncSetAttribute(k_ref_cfmat, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(sizeof(double) * kCfSm));
-  if (e) return e;
-  k_ref_cfmat<<<c->rg.nnpinv, kCfThreads, sizeof(double) * kCfSm, st>>>(
-      c->mv, c->dt, ra, c->d_lm, c->d_rg_anchor, c->d_mconn, c->d_elem_wts, c->d_jcsc, c->d_icsc,
-      (const float2 *)wave, c->d_fmat, c->d_err);
-  return cudaGetLastError();
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+  // figures at the kernel: an SM for every anchor, or operations that count
+  return c->rg.nnpinv <= nsm ? ref_cfmat<1>(c, ra, wave, st) : ref_cfmat<kNl>(c, ra, wave, st);
 }
 
 static size_t vforce2_smem() {
