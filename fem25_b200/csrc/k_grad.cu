@@ -29,7 +29,8 @@
 // SM; the next tile's fields arrive by cp.async while this one is computed.
 // 12 000 elements, 64 (pair, source) fields: 3.6 ms against 13.2 ms with the full
 // table (1 224 bytes of field per element and source would take 0.2 ms); the
-// shared-memory pipe is then 75 % busy and the FP64 pipe 53 %.
+// shared-memory pipe is then 75 % busy and the FP64 pipe 53 %.  The forms of both
+// points at once fill the 168 registers that four CTAs leave (64 bytes of stack).
 #include <cstdlib>
 
 #include "ctx.cuh"

@@ -1203,10 +1203,10 @@ cudaError_t sparse_factor_level(SparseLU *s, int l, const double2 *csr, double2 
         ne, s->d_ent_idx + s->lev_ent0[l], s->d_ent_loc + s->lev_ent0[l], csr, W);
   // The fronts in groups, each on a stream of its own: a group's pivot searches (one
   // CTA a front) run beside another's products, and within a group the next panel
-  // beside the update of the columns behind it.  Before F22's sums moved into the
-  // products (the line above k_sp_pull): 38.7 ms on one stream, 37.4 in
+  // beside the update of the columns behind it.  A factorisation of 331 GFLOP and a
+  // solve, measured while k_sp_pull still wrote F22: 38.7 ms on one stream, 37.4 in
   // groups, 36.2 with the side streams, 35.7 with the groups' streams first in
-  // priority (2 to 4 groups within 1 %, 8 slower).
+  // priority (2 to 4 groups within 1 %, 8 slower); 34.7 now.
   cudaError_t e;
   const int groups = std::min(sp::kStreams, nfl);
   if ((e = cudaEventRecord(s->ready, st))) return e;
